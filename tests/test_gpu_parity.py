@@ -594,3 +594,39 @@ def test_oc_update_exact_volume(native, oracle, n, move):
     assert nb == nbr and lm == lmr
     assert np.array_equal(xn, xr)
     assert ch == np.abs(xr.astype(np.float64) - x.astype(np.float64)).max()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dims,kind", [((1, 1, 1), "plain"), ((31, 33, 1), "plain"), ((32, 32, 1), "masks"),
+                                       ((25, 41, 1), "masks"), ((60, 20, 20), "signs"), ((256, 128, 120), "masks")])
+def test_oc_bisect_edges(native, oracle, dims, kind):
+    """The one-launch bisection at its edges: one element, one element below and at a full
+    block, one above it, several blocks, and more elements per block than its shared memory
+    holds (3.9M).  'masks': preserved and void elements; 'signs': zero, infinite and NaN
+    sensitivities, and a positive one (NaN in the reference).  Bit for bit against the
+    oracle, as the sum is exact."""
+    import torch
+    from topologyoptimization_b200 import Problem, mesh
+    n = int(np.prod(dims))
+    rng = np.random.default_rng(n)
+    x = rng.uniform(0, 1, n).astype(np.float32)
+    dc = (-(10.0 ** rng.uniform(-9, 5, n))).astype(np.float32)
+    pres = void = None
+    if kind == "masks":
+        pres, void = (rng.random(n) < 0.1).astype(np.uint8), (rng.random(n) < 0.1).astype(np.uint8)
+    if kind == "signs":
+        dc[:64] = 0.0
+        dc[64:80] = -np.inf
+        x[80:90] = 0.0
+        dc[85:95] = -np.inf
+        dc[100] = np.nan
+        dc[200] = 1.0
+    with np.errstate(all="ignore"):
+        xr, lmr, nbr = oracle.oc(x, 0.3, dc, preserved=pres, void=void)
+    with Problem(*dims, mesh.fixed_mask(*dims, "left")) as P:
+        d = [None if m is None else _dev(m) for m in (pres, void)]
+        d_xn = torch.empty(n, dtype=torch.float32, device="cuda")
+        ch, lm, nb = P.oc_update_dev(_dev(x), _dev(dc), d_xn, 0.3, d_preserved=d[0], d_void=d[1])
+        xn = d_xn.cpu().numpy()
+    assert nb == nbr and lm == lmr
+    assert np.array_equal(xn, xr, equal_nan=True)

@@ -1574,53 +1574,54 @@ void ensure_simp_arrays(tpo_problem *P) {
     CK(cudaMemset(P->stress_max, 0, sizeof(unsigned long long)));
 }
 
-// Device state of one OC bisection: stream, bisection state (device and pinned host copy),
-// reduction partials and the change scalar.
+// Device state of one OC bisection: stream, bisection state (device and pinned host copy)
+// and the words the blocks publish.
 struct OcCtx {
     cudaStream_t s;
     OCState *oc, *oc_host;
-    double *partials, *scal, *scal_host;
+    double *partials;
     long long n;
 };
 
+// One cooperative launch: a block of kOcThreads per SM at most, each keeping as many of its
+// elements as fit in shared memory.
 void run_oc_ctx(const OcCtx &c, const float *d_x, double volfrac, const float *d_dc, const uint8_t *pres,
                 const uint8_t *voidm, float *d_xnew, const float *d_xold, double *lmid, int *nb, double *change,
                 double move, int max_bisections) {
-    k_oc_init<<<1, 32, 0, c.s>>>(c.oc);
+    int dev = 0, sms = 0, optin = 0;
+    CK(cudaGetDevice(&dev));
+    CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    const long long blocks = std::max(1LL, std::min<long long>(std::min(sms, 1024), (c.n + kOcThreads - 1) / kOcThreads));
+    long long per = (c.n + blocks - 1) / blocks;
+    if (per >= (1LL << 31)) fail(TPO_BAD_ARG, "too many elements for the OC update");
+    const size_t room = (size_t)std::max(optin - 8 * 1024, 0);  // beside the kernel's static arrays
+    int cap = (int)std::min<long long>(per, (long long)(room / sizeof(float2)));
+    const size_t smem = (size_t)cap * sizeof(float2);
+    CK(cudaFuncSetAttribute(k_oc_bisect, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)room));
+    CK(cudaMemsetAsync(c.oc, 0, sizeof(OCState), c.s));
+    long long n = c.n;
+    OCState *oc = c.oc;
+    unsigned long long *words = reinterpret_cast<unsigned long long *>(c.partials);
+    void *args[] = {&d_x, &d_dc, &pres, &voidm, &n, &per, &cap, &volfrac, &move, &max_bisections, &oc, &words, &d_xold, &d_xnew};
+    CK(cudaLaunchCooperativeKernel((const void *)k_oc_bisect, dim3((unsigned)blocks), dim3(kOcThreads), args, smem, c.s));
     CKL();
-    int launched = 0;
-    while (launched < max_bisections) {
-        const int chunk = std::min(16, max_bisections - launched);
-        for (int i = 0; i < chunk; i++) {
-            k_oc_step<<<red_blocks(), 256, 0, c.s>>>(d_x, d_dc, pres, voidm, c.n, volfrac, move, c.oc, c.partials);
-            CKL();
-        }
-        launched += chunk;
-        CK(cudaMemcpyAsync(c.oc_host, c.oc, sizeof(OCState), cudaMemcpyDeviceToHost, c.s));
-        CK(cudaStreamSynchronize(c.s));
-        if (c.oc_host->done) break;
-    }
+    CK(cudaMemcpyAsync(c.oc_host, c.oc, sizeof(OCState), cudaMemcpyDeviceToHost, c.s));
+    CK(cudaStreamSynchronize(c.s));
+    if (c.oc_host->err) fail(TPO_TIMEOUT, "a grid barrier of the OC bisection ran out");
     if (!c.oc_host->done)
         fail(TPO_TIMEOUT, "OC bisection did not terminate within " + std::to_string(max_bisections) + " steps");
-    unsigned long long *bits = reinterpret_cast<unsigned long long *>(&c.scal[1]);
-    CK(cudaMemsetAsync(bits, 0, sizeof(unsigned long long), c.s));
-    k_oc_write<<<red_blocks(), 256, 0, c.s>>>(d_x, d_dc, pres, voidm, c.n, move, c.oc, d_xold, d_xnew,
-                                              d_xold ? bits : nullptr);
-    CKL();
-    CK(cudaMemcpyAsync(c.scal_host, c.scal, 2 * sizeof(double), cudaMemcpyDeviceToHost, c.s));
-    CK(cudaStreamSynchronize(c.s));
     if (lmid) *lmid = c.oc_host->last_lmid;
     if (nb) *nb = c.oc_host->nb;
-    if (change) *change = c.scal_host[1];
+    if (change) std::memcpy(change, &c.oc_host->change_bits, sizeof(double));
 }
 
-// OC (js/optimizer-worker-3d.js:3066-3101): device bisection, the host polling every 16
-// steps; more than max_bisections steps (the reference's loop ends within ~1100 halvings
-// even in degenerate cases) returns TPO_TIMEOUT.
+// OC (js/optimizer-worker-3d.js:3066-3101); more than max_bisections steps (the reference's
+// loop ends within ~1100 halvings even in degenerate cases) returns TPO_TIMEOUT.
 void run_oc(tpo_problem *P, const float *d_x, double volfrac, const float *d_dc, const uint8_t *pres,
             const uint8_t *voidm, float *d_xnew, const float *d_xold, double *lmid, int *nb, double *change,
             double move = 0.2, int max_bisections = 1280) {
-    const OcCtx c{P->s, P->oc, P->oc_host, P->partials, P->scal, P->scal_host, P->g.nel};
+    const OcCtx c{P->s, P->oc, P->oc_host, P->partials, P->g.nel};
     run_oc_ctx(c, d_x, volfrac, d_dc, pres, voidm, d_xnew, d_xold, lmid, nb, change, move, max_bisections);
 }
 
@@ -2857,7 +2858,7 @@ tpo_status tpo_simp2d_step_dev(tpo_problem2d *p, const tpo_simp2d_opts *o, float
         CK(cudaStreamSynchronize(s));
         const double compliance = p->scal_host[0];
         double change = 0.0;
-        const OcCtx c{s, p->oc, p->oc_host, p->partials, p->scal, p->scal_host, ne};
+        const OcCtx c{s, p->oc, p->oc_host, p->partials, ne};
         run_oc_ctx(c, p->xold, o->volfrac, p->dcn, d_preserved, d_void, d_x, p->xold, nullptr, nullptr, &change, 0.2,
                    1280);
         if (info) {

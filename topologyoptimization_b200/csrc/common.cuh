@@ -225,6 +225,29 @@ __device__ __forceinline__ bool grid_sum(double (&v)[NV], double *partials, unsi
     return true;
 }
 
+// ---- grid barrier of a cooperative launch ---------------------------------------
+// Every block arrives once per epoch; `target` is epoch * blocks.  All blocks are resident (a
+// cooperative launch), so the wait ends; a wait of some seconds sets *err instead, and the
+// kernel returns.  What a block wrote before the barrier is visible to every block after it
+// (reads of such data use __ldcg or volatile accesses: L1 is not coherent).
+constexpr unsigned kBarrierSpins = 1u << 22;
+__device__ __forceinline__ bool grid_barrier(unsigned *count, unsigned target, int *err) {
+    __shared__ int s_ok;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        atomicAdd(count, 1u);
+        unsigned v, spins = 0;
+        do {
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(count) : "memory");
+        } while ((int)(v - target) < 0 && ++spins < kBarrierSpins);
+        s_ok = (int)(v - target) >= 0;
+        if (!s_ok) atomicExch(err, 1);
+    }
+    __syncthreads();
+    return s_ok != 0;
+}
+
 // ---- cp.async (8-byte and 4-byte), zero fill when src_bytes == 0 --------------
 __device__ __forceinline__ void cp_async8(void *smem, const void *gmem, bool valid) {
     const unsigned s = (unsigned)__cvta_generic_to_shared(smem);

@@ -489,82 +489,172 @@ __device__ double x192_to_double(const Exact192 &a) {
     return ldexp((double)mant, sh - 149);
 }
 
-__global__ void k_oc_init(OCState *s) {
-    if (threadIdx.x || blockIdx.x) return;
-    s->l1 = 0.0;
-    s->l2 = 1e9;
-    s->lmid = 0.0;
-    s->last_lmid = 0.0;
-    s->sum = 0.0;
-    s->nb = 0;
-    s->counter = 0u;
-    s->done = !((s->l2 - s->l1) / (s->l2 + s->l1) > 1e-3);
+// ---- the whole bisection in one cooperative launch ---------------------------------------
+// A value's sum in units of 2^-51: v in [2^-28, 2) is a multiple of 2^-51, and the bits of
+// v + 2.0 minus those of 2.0 are v 2^51 (same binade, no rounding).  2^51 times 4096 values
+// below 2 stays inside 64 bits.
+constexpr int kFastFlush = 4096;
+
+__device__ __forceinline__ void x192_add_u51(Exact192 &a, unsigned long long u) {
+    // u 2^-51 = u 2^98 2^-149: limb 1, offset 34
+    const Exact192 t{0ULL, u << 34, u >> 30, 0u};
+    x192_add(a, t);
 }
 
-// One bisection step: lmid = (l1 + l2)/2, sum xnew(lmid) exactly, move the bracket
-// (OC, js/optimizer-worker-3d.js:3066-3101).  partials holds 4 words per block.
-__global__ void k_oc_step(const float *__restrict__ x, const float *__restrict__ dc,
-                          const uint8_t *__restrict__ pres, const uint8_t *__restrict__ voidm, long long n,
-                          double volfrac, double move, OCState *s, double *partials) {
-    if (s->done) return;
-    const double lmid = 0.5 * (s->l2 + s->l1);
-    Exact192 acc{0ULL, 0ULL, 0ULL, 0u};
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-        x192_add_float(acc, oc_xnew(x[i], dc[i], pres, voidm, i, lmid, move));
+// Sum over the block in thread 0.
+__device__ __forceinline__ Exact192 x192_block_sum(Exact192 acc, Exact192 *sh) {
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         const Exact192 b = x192_shfl_down(acc, o);
         x192_add(acc, b);
     }
-    __shared__ Exact192 sh[32];
-    __shared__ bool s_last;
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     if (lane == 0) sh[wid] = acc;
     __syncthreads();
-    unsigned long long *pw = reinterpret_cast<unsigned long long *>(partials);
-    if (threadIdx.x == 0) {
-        Exact192 b{0ULL, 0ULL, 0ULL, 0u};
-        for (int w = 0; w < (int)(blockDim.x >> 5); w++) x192_add(b, sh[w]);
-        pw[4 * blockIdx.x + 0] = b.w0;
-        pw[4 * blockIdx.x + 1] = b.w1;
-        pw[4 * blockIdx.x + 2] = b.w2;
-        pw[4 * blockIdx.x + 3] = b.nan;
-        __threadfence();
-        const unsigned int t = atomicAdd(&s->counter, 1u);
-        s_last = (t == gridDim.x - 1);
+    if (wid == 0) {
+        acc = lane < nw ? sh[lane] : Exact192{0ULL, 0ULL, 0ULL, 0u};
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const Exact192 b = x192_shfl_down(acc, o);
+            x192_add(acc, b);
+        }
     }
-    __syncthreads();
-    if (!s_last || threadIdx.x != 0) return;
-    __threadfence();
-    Exact192 tot{0ULL, 0ULL, 0ULL, 0u};
-    for (unsigned b = 0; b < gridDim.x; b++) {
-        const Exact192 pb{__ldcg(&pw[4 * b + 0]), __ldcg(&pw[4 * b + 1]), __ldcg(&pw[4 * b + 2]),
-                          (unsigned int)__ldcg(&pw[4 * b + 3])};
-        x192_add(tot, pb);
-    }
-    s->counter = 0u;
-    const double sum = x192_to_double(tot);
-    s->sum = sum;
-    s->last_lmid = lmid;
-    if (sum > volfrac * (double)n) s->l1 = lmid;
-    else s->l2 = lmid;
-    s->nb += 1;
-    if (!((s->l2 - s->l1) / (s->l2 + s->l1) > 1e-3)) s->done = 1;
+    return acc;
 }
 
-// xnew at the last evaluated lmid; change = max |xnew - xold| (exact, order-free max).
-__global__ void k_oc_write(const float *__restrict__ x, const float *__restrict__ dc,
-                           const uint8_t *__restrict__ pres, const uint8_t *__restrict__ voidm, long long n,
-                           double move, const OCState *s, const float *__restrict__ xold, float *__restrict__ xnew,
-                           unsigned long long *change_bits) {
-    const double lmid = s->last_lmid;
-    double mx = 0.0;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const float v = oc_xnew(x[i], dc[i], pres, voidm, i, lmid, move);
-        xnew[i] = v;
-        if (xold) mx = js_max(mx, fabs((double)v - (double)xold[i]));
+// xnew(lmid) of one element as oc_xnew forms it.  rl = 1 / lmid in FP32: an FP32 estimate of
+// s = x sqrt(-dc / lmid) (relative error below 1e-6 in the range tested) decides an element
+// that lies clear of the move limits, where the result is the limit itself; the others, and
+// every value outside the estimate's range (NaN included), take the FP64 division and root.
+__device__ __forceinline__ float oc_xnew_fast(float xf, float dcf, double lmid, float rl, double move) {
+    const double x = (double)xf, lo = x - move, hi = x + move;
+    const float bf = -dcf * rl;
+    if (bf < 1e30f) {
+        const float sf = xf * sqrtf(bf);
+        const float hf = fminf((float)hi, 1.0f), lf = (float)lo;
+        if (sf > hf * 1.00001f && sf < 1e30f && hf > 1e-6f) return (float)js_max(0.0, js_max(lo, js_min(1.0, hi)));
+        if (sf < lf * 0.99999f && lf > 1e-6f) return (float)js_max(0.0, js_max(lo, js_min(1.0, lo)));
     }
-    if (change_bits) {
+    return oc_xnew(xf, dcf, nullptr, nullptr, 0, lmid, move);
+}
+
+// OC (js/optimizer-worker-3d.js:3066-3101): bisection on the multiplier, then xnew at the last
+// one and change = max |xnew - xold|.  Block b owns elements [b per, (b + 1) per); it keeps the
+// first `cap` of them (x, dc) in shared memory for all steps.  Each step every block sums its
+// xnew exactly, publishes the four words, passes the grid barrier and adds up all blocks'
+// words itself (integers: the same total everywhere), so a step costs one barrier.  Preserved
+// and void elements contribute a constant, added once.  partials: 2 x 4 words per block.
+//
+// One launch per step, each with its last block adding the partials of 592 blocks in one
+// thread, took 47-54 us a step whatever the size (24,000 to 2,000,000 elements): the serial
+// sum.  Here a step is bound by the barrier (about 2.5 us) up to 100,000 elements and by the
+// per-element arithmetic beyond.
+__global__ void __launch_bounds__(kOcThreads) k_oc_bisect(const float *x, const float *dc,
+                                                          const uint8_t *__restrict__ pres,
+                                                          const uint8_t *__restrict__ voidm, long long n, long long per,
+                                                          int cap, double volfrac, double move, int max_bisections,
+                                                          OCState *s, unsigned long long *partials, const float *xold,
+                                                          float *xnew) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    float2 *sv = reinterpret_cast<float2 *>(smem_raw);
+    __shared__ Exact192 sh[32];
+    __shared__ double s_l[3];
+    __shared__ int s_done;
+    const long long b0 = blockIdx.x * per, b1 = min(n, b0 + per);
+    const int ne = (int)max(0LL, b1 - b0);
+    const int ns = min(ne, cap);
+    Exact192 base{0ULL, 0ULL, 0ULL, 0u};  // preserved elements: 1 each
+    // masked elements enter the loop as x = dc = 0, whose xnew is 0
+    auto load = [&](int i) {
+        const long long e = b0 + i;
+        return (pres && pres[e]) || (voidm && voidm[e]) ? make_float2(0.f, 0.f) : make_float2(x[e], dc[e]);
+    };
+    for (int i = threadIdx.x; i < ne; i += blockDim.x)
+        if (pres && pres[b0 + i]) x192_add_u51(base, 1ULL << 51);
+    for (int i = threadIdx.x; i < ns; i += blockDim.x) sv[i] = load(i);
+    __syncthreads();
+    double l1 = 0.0, l2 = 1e9, lmid = 0.0, sum = 0.0;
+    int nb = 0;
+    bool done = !((l2 - l1) / (l2 + l1) > 1e-3);
+    while (!done && nb < max_bisections) {
+        lmid = 0.5 * (l2 + l1);
+        const float rl = (float)(1.0 / lmid);
+        Exact192 acc = base;
+        unsigned long long fast = 0ULL;
+        int nf = 0;
+        auto add = [&](float2 v) {
+            const float r = oc_xnew_fast(v.x, v.y, lmid, rl, move);
+            if (r >= 0x1p-28f && r < 2.0f) {
+                fast += (unsigned long long)(__double_as_longlong((double)r + 2.0) - 0x4000000000000000LL);
+                if (++nf == kFastFlush) {
+                    x192_add_u51(acc, fast);
+                    fast = 0ULL;
+                    nf = 0;
+                }
+            } else if (r != 0.0f) {
+                x192_add_float(acc, r);
+            }
+        };
+        for (int i = threadIdx.x; i < ns; i += blockDim.x) add(sv[i]);
+        for (int i = ns + threadIdx.x; i < ne; i += blockDim.x) add(load(i));
+        x192_add_u51(acc, fast);
+        __syncthreads();  // sh is free (the previous step's readers are past it)
+        acc = x192_block_sum(acc, sh);
+        unsigned long long *pw = partials + (size_t)(nb & 1) * 4 * gridDim.x;
+        if (threadIdx.x == 0) {
+            pw[4 * blockIdx.x + 0] = acc.w0;
+            pw[4 * blockIdx.x + 1] = acc.w1;
+            pw[4 * blockIdx.x + 2] = acc.w2;
+            pw[4 * blockIdx.x + 3] = acc.nan;
+        }
+        if (!grid_barrier(&s->bar, (unsigned)(nb + 1) * gridDim.x, &s->err)) return;
+        if (threadIdx.x < 32) {
+            Exact192 tot{0ULL, 0ULL, 0ULL, 0u};
+            for (unsigned b = threadIdx.x; b < gridDim.x; b += 32) {
+                const Exact192 pb{__ldcg(&pw[4 * b + 0]), __ldcg(&pw[4 * b + 1]), __ldcg(&pw[4 * b + 2]),
+                                  (unsigned int)__ldcg(&pw[4 * b + 3])};
+                x192_add(tot, pb);
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                const Exact192 b = x192_shfl_down(tot, o);
+                x192_add(tot, b);
+            }
+            if (threadIdx.x == 0) {
+                const double t = x192_to_double(tot);
+                if (t > volfrac * (double)n) l1 = lmid;
+                else l2 = lmid;
+                s_l[0] = l1;
+                s_l[1] = l2;
+                s_l[2] = t;
+                s_done = !((l2 - l1) / (l2 + l1) > 1e-3);
+            }
+        }
+        __syncthreads();
+        l1 = s_l[0];
+        l2 = s_l[1];
+        sum = s_l[2];
+        done = s_done != 0;
+        nb++;
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        s->l1 = l1;
+        s->l2 = l2;
+        s->lmid = s->last_lmid = lmid;
+        s->sum = sum;
+        s->nb = nb;
+        s->done = done;
+    }
+    if (!done) return;
+    // xnew at the last evaluated lmid; change = max |xnew - xold| (exact, order-free max)
+    double mx = 0.0;
+    for (int i = threadIdx.x; i < ne; i += blockDim.x) {
+        const long long e = b0 + i;
+        const float v = oc_xnew(x[e], dc[e], pres, voidm, e, lmid, move);
+        if (xold) mx = js_max(mx, fabs((double)v - (double)xold[e]));
+        xnew[e] = v;
+    }
+    if (xold) {
         // non-negative doubles order like their bit patterns
         unsigned long long b = (unsigned long long)__double_as_longlong(mx);
 #pragma unroll
@@ -572,7 +662,7 @@ __global__ void k_oc_write(const float *__restrict__ x, const float *__restrict_
             const unsigned long long ob = __shfl_xor_sync(0xffffffffu, b, o);
             b = ob > b ? ob : b;
         }
-        if ((threadIdx.x & 31) == 0) atomicMax(change_bits, b);
+        if ((threadIdx.x & 31) == 0) atomicMax(&s->change_bits, b);
     }
 }
 

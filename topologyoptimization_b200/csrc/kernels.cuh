@@ -4,11 +4,15 @@
 
 namespace tpo {
 
+// Bracket and result of one OC bisection; zeroed before the launch.
 struct OCState {
     double l1, l2, lmid, last_lmid, sum;
+    unsigned long long change_bits;  // max |xnew - xold| as the bits of a non-negative double
     int done, nb;
-    unsigned int counter;
+    unsigned int bar;  // arrivals at the launch's grid barrier
+    int err;           // the barrier's wait ran out
 };
+constexpr int kOcThreads = 1024;
 
 // element stiffness
 __global__ void k_lk(double nu, double *Ke);
@@ -107,20 +111,18 @@ __global__ void k_filter_sens_tiled(Grid g, double rmin, const float *__restrict
                                     const float *__restrict__ dc, float *__restrict__ dcn);
 __global__ void k_density_tiled(Grid g, double radius, int mode, const double *__restrict__ in,
                                 double *__restrict__ out);
-__global__ void k_oc_init(OCState *s);
 // adjoint: dJ/dxPhys (reference order) and the density-filter transpose
 __global__ void k_adjoint_sens(const __grid_constant__ KeParam<double> ke, Grid g, const double *__restrict__ xphys,
                                const double *__restrict__ U, const double *__restrict__ Lam, double penal, double E0,
                                double Emin, double *__restrict__ out);
 __global__ void k_density_scale(Grid g, double radius, const double *__restrict__ gin, double *__restrict__ t);
 __global__ void k_density_stencil(Grid g, double radius, const double *__restrict__ t, double *__restrict__ out);
-__global__ void k_oc_step(const float *__restrict__ x, const float *__restrict__ dc,
-                          const uint8_t *__restrict__ pres, const uint8_t *__restrict__ voidm, long long n,
-                          double volfrac, double move, OCState *s, double *partials);
-__global__ void k_oc_write(const float *__restrict__ x, const float *__restrict__ dc,
-                           const uint8_t *__restrict__ pres, const uint8_t *__restrict__ voidm, long long n,
-                           double move, const OCState *s, const float *__restrict__ xold,
-                           float *__restrict__ xnew, unsigned long long *change_bits);
+__global__ void __launch_bounds__(kOcThreads) k_oc_bisect(const float *x, const float *dc,
+                                                          const uint8_t *__restrict__ pres,
+                                                          const uint8_t *__restrict__ voidm, long long n, long long per,
+                                                          int cap, double volfrac, double move, int max_bisections,
+                                                          OCState *s, unsigned long long *partials, const float *xold,
+                                                          float *xnew);
 
 __global__ void k_energy_wgsl(const float *__restrict__ U, const float *__restrict__ KE,
                               const int32_t *__restrict__ edofs, int nel, int es, float *__restrict__ out);
