@@ -630,3 +630,24 @@ def test_oc_bisect_edges(native, oracle, dims, kind):
         xn = d_xn.cpu().numpy()
     assert nb == nbr and lm == lmr
     assert np.array_equal(xn, xr, equal_nan=True)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dims", [(4, 4, 4), (5, 5, 5), (7, 4, 11), (21, 13, 9), (60, 20, 20)])
+def test_galerkin_stencil_bitwise(native, oracle, dims):
+    """Every dense level at the smallest grid with one, odd sizes on each axis and the largest
+    first dense level below 3000 DOFs of a worker's grid: bit for bit the oracle's, zeros
+    outside the 27-point stencil included."""
+    from topologyoptimization_b200 import Problem, mesh
+    fixed = mesh.fixed_mask(*dims, "left")
+    rng = np.random.default_rng(5)
+    x = rng.uniform(0.2, 1.0, int(np.prod(dims))).astype(np.float32)
+    x[rng.random(x.size) < 0.2] = 1e-3  # inactive elements
+    mg = oracle.MG(*dims, oracle.lk(0.3), fixed)
+    mg.update(x, 3.0)
+    with Problem(*dims, fixed) as P:
+        P.set_densities(x, 3.0)
+        dense = [li for li in range(1, P.levels) if P.level_info(li)["dense"]]
+        assert dense
+        for li in dense:
+            assert np.array_equal(P.level_dense(li), mg.level_arrays(li)[2]), li

@@ -728,6 +728,7 @@ void build_levels(tpo_problem *P) {
         }
         if (L.dense) {
             L.K = dalloc<double>((size_t)g.ndof * g.ndof);
+            CK(cudaMemset(L.K, 0, (size_t)g.ndof * g.ndof * sizeof(double)));
             if (P->L[li - 1].dense) maxT = std::max(maxT, (size_t)(P->L[li - 1].g.ndof * g.ndof));
         }
     }
@@ -833,7 +834,8 @@ void build_hierarchy(tpo_problem *P, double Emin) {
                 k_galerkin_PtT<<<nblk(n * n), 256, 0, s>>>(Lf.g, L.g, P->Ttmp, L.K);
                 CKL();
             } else {
-                k_galerkin_gather<<<nblk(n * n), 256, 0, s>>>(P->ke, Lf.g, L.g, Lf.Eact, L.K);
+                // entries outside the stencil stay at the zero they were created with
+                k_galerkin_gather<<<nblk(243 * L.g.nnodes, 128), 128, 0, s>>>(P->ke, Lf.g, L.g, Lf.Eact, L.K);
                 CKL();
             }
             k_dense_invdiag<<<nblk(n), 256, 0, s>>>(L.K, (int)n, L.fixed, L.invD, L.invD32);

@@ -31,8 +31,9 @@ __global__ void k_diag(const __grid_constant__ KeParam<double> ke, Grid g, const
 
 // dense coarse levels
 __global__ void k_zero_d(double *a, long long n);
-__global__ void k_galerkin_gather(const __grid_constant__ KeParam<double> ke, Grid gf, Grid gc,
-                                  const double *__restrict__ EactF, double *__restrict__ Kc);
+// one thread per entry of the coarse 27-point stencil (243 per coarse node)
+__global__ void __launch_bounds__(128) k_galerkin_gather(const __grid_constant__ KeParam<double> ke, Grid gf, Grid gc,
+                                                         const double *__restrict__ EactF, double *__restrict__ Kc);
 __global__ void k_galerkin_T(Grid gf, Grid gc, const double *__restrict__ Kf, double *__restrict__ T);
 __global__ void k_galerkin_PtT(Grid gf, Grid gc, const double *__restrict__ T, double *__restrict__ Kc);
 __global__ void k_dense_invdiag(const double *__restrict__ K, int n, const uint8_t *__restrict__ fixed,
