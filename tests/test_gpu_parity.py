@@ -651,3 +651,29 @@ def test_galerkin_stencil_bitwise(native, oracle, dims):
         assert dense
         for li in dense:
             assert np.array_equal(P.level_dense(li), mg.level_arrays(li)[2]), li
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dims,kw", [((4, 4, 4), {}), ((5, 4, 7), dict(nu1=0)), ((16, 8, 8), dict(nu1=1, coarse_iters=2)),
+                                     ((16, 8, 8), dict(nu1=3, coarse_iters=4)), ((30, 10, 10), {}),
+                                     ((64, 32, 32), dict(max_levels=4)), ((34, 18, 18), dict(max_levels=3))])
+def test_vcycle_dense_levels(native, oracle, dims, kw):
+    """V-cycles whose dense levels take each of their forms: the coarsest level's sweeps as a
+    matrix (27, 81, 216 and 675 DOFs), as launches (fewer than four; 810 DOFs is above the
+    matrix's limit), the first two sweeps of a dense level in one launch or not (nu1 = 0, 1, 2,
+    3).  FP64 sums in another order: within 1e-11 of the oracle, as the other V-cycle tests."""
+    from topologyoptimization_b200 import Problem, mesh
+    fixed = mesh.fixed_mask(*dims, "left")
+    x = np.random.default_rng(8).uniform(0.3, 1.0, int(np.prod(dims))).astype(np.float32)
+    b = np.random.default_rng(9).standard_normal(len(fixed)) * (fixed == 0)
+    mg = oracle.MG(*dims, oracle.lk(0.3), fixed, **kw)
+    mg.update(x, 3.0)
+    with Problem(*dims, fixed, mg=native.default_mg_opts(**kw)) as P:
+        P.set_densities(x, 3.0)
+        z = P.vcycle(b)
+        P.set_densities(1.0 - 0.5 * x, 2.0)  # the matrix follows the moduli
+        z2 = P.vcycle(b)
+    zo = mg.vcycle(b)
+    mg.update(1.0 - 0.5 * x, 2.0)
+    assert rel_inf(z, zo) < 1e-11
+    assert rel_inf(z2, mg.vcycle(b)) < 1e-11

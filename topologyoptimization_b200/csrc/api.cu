@@ -525,6 +525,10 @@ struct Level {
     double cheb_w0 = 0.0;
     std::vector<double> cheb_cd, cheb_cr;
     double *womega = nullptr;   // dense levels under safe_omega: damping set on the device
+    // coarsest level without a direct solve: its sweeps from zero as a matrix, for the moduli of
+    // S_version (formed when a V-cycle first needs it)
+    double *S = nullptr, *Sk = nullptr;
+    long long S_version = -1;
 };
 
 }  // namespace
@@ -638,7 +642,7 @@ void problem_free(tpo_problem *P) {
         dfree(L.fixed); dfree(L.E); dfree(L.Eact); dfree(L.invD); dfree(L.Eact32); dfree(L.invD32);
         dfree(L.b); dfree(L.x); dfree(L.xt); dfree(L.res); dfree(L.K);
         dfree(L.b32); dfree(L.x32); dfree(L.xt32); dfree(L.res32);
-        dfree(L.Kinv); dfree(L.Lw); dfree(L.Yw); dfree(L.womega);
+        dfree(L.Kinv); dfree(L.Lw); dfree(L.Yw); dfree(L.womega); dfree(L.S); dfree(L.Sk);
         if (L.gj) cudaGraphExecDestroy(L.gj);
     }
     dfree(P->U); dfree(P->F); dfree(P->r); dfree(P->z); dfree(P->p); dfree(P->Ap); dfree(P->partials);
@@ -733,6 +737,17 @@ void build_levels(tpo_problem *P) {
         }
     }
     if (maxT) P->Ttmp = dalloc<double>(maxT);
+    {
+        // Sweeps as a matrix: from 4 sweeps on, up to kPolyMaxN DOFs (675, the coarsest level of
+        // a 256x128x128 grid), where forming it stays below the time of five V-cycles' sweeps.
+        Level &C = P->L[P->nl - 1];
+        if (C.dense && !o.coarse_direct && o.nu1 + o.coarse_iters >= 4 && C.g.ndof <= kPolyMaxN) {
+            C.S = dalloc<double>((size_t)C.g.ndof * C.g.ndof);
+            C.Sk = dalloc<double>((size_t)81 * C.g.ndof);
+            CK(cudaFuncSetAttribute(k_coarse_poly, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)coarse_poly_smem(kPolyMaxN)));
+        }
+    }
     if (o.coarse_direct) {
         Level &C = P->L[P->nl - 1];
         if (!C.dense)
@@ -769,13 +784,16 @@ void build_levels(tpo_problem *P) {
     // kappa(Ke) = lambda_max(diag(Ke)^-1 Ke) bounds lambda_max(D^-1 A) for any moduli
     // (A and D are both sums of E_e Ke over the elements), so the smoother converges and
     // the symmetric V-cycle stays positive definite; dense levels get theirs on the device
-    // from a Gershgorin bound at every hierarchy update (k_dense_jacobi_bound).
+    // from a Gershgorin bound at every hierarchy update (k_dense_rows).
     const double kappa = (o.safe_omega || o.chebyshev) ? jacobi_kappa(P->Ke) : 0.0;
     for (int li = 0; li < P->nl; li++) {
         Level &L = P->L[li];
         L.omega = o.omega;
         if (o.safe_omega && !L.dense) L.omega = std::min(o.omega, 1.9 / kappa);
-        if (o.safe_omega && L.dense) L.womega = dalloc<double>(1);
+        if (o.safe_omega && L.dense) {
+            L.womega = dalloc<double>(3);
+            CK(cudaMemset(L.womega, 0, 3 * sizeof(double)));
+        }
         if (o.chebyshev && !L.dense) {
             // Chebyshev iteration on [kappa / ratio, kappa] (Adams et al. 2003): theta and
             // delta the interval's centre and half width, sigma = theta / delta, rho_0 =
@@ -838,12 +856,8 @@ void build_hierarchy(tpo_problem *P, double Emin) {
                 k_galerkin_gather<<<nblk(243 * L.g.nnodes, 128), 128, 0, s>>>(P->ke, Lf.g, L.g, Lf.Eact, L.K);
                 CKL();
             }
-            k_dense_invdiag<<<nblk(n), 256, 0, s>>>(L.K, (int)n, L.fixed, L.invD, L.invD32);
+            k_dense_rows<<<nblk(n, 8), 256, 0, s>>>(L.K, L.g, L.fixed, P->mg.omega, L.invD, L.invD32, L.womega);
             CKL();
-            if (L.womega) {
-                k_dense_jacobi_bound<<<1, 256, 0, s>>>(L.K, (int)n, L.fixed, P->mg.omega, L.womega);
-                CKL();
-            }
             if (L.Kinv) {  // coarsest level with a direct solve: explicit inverse by n sweeps
                 k_coarse_prepare<<<nblk(n * n), 256, 0, s>>>(L.K, (int)n, L.invD, L.Lw);
                 CKL();
@@ -980,9 +994,8 @@ void smooth(tpo_problem *P, int li, const T *b, const T *x, T *xn, const CGState
             bool from_zero = false) {
     Level &L = P->L[li];
     if (L.dense) {
-        const int n = (int)L.g.ndof;
-        k_dense_smooth<T><<<G(P, (n + 7) / 8), 256, 0, P->s>>>(L.K, n, x, b, Prec<T>::invD(L), L.fixed, (T)L.omega,
-                                                          L.womega, xn, st);
+        k_dense_smooth<T><<<G(P, nblk(L.g.ndof, 8)), 256, 0, P->s>>>(L.K, L.g, x, b, Prec<T>::invD(L), L.fixed,
+                                                                    (T)L.omega, L.womega, xn, st);
         CKL();
     } else if (L.cheb && k > 0) {
         if (k >= (int)L.cheb_cd.size()) fail(TPO_BAD_ARG, "Chebyshev sweep beyond the level's coefficients");
@@ -1011,8 +1024,7 @@ template <typename T>
 void residual(tpo_problem *P, int li, const T *b, const T *x, T *res, const CGState *st) {
     Level &L = P->L[li];
     if (L.dense) {
-        const int n = (int)L.g.ndof;
-        k_dense_residual<T><<<G(P, (n + 7) / 8), 256, 0, P->s>>>(L.K, n, x, b, L.fixed, res, st);
+        k_dense_residual<T><<<G(P, nblk(L.g.ndof, 8)), 256, 0, P->s>>>(L.K, L.g, x, b, L.fixed, res, st);
         CKL();
     } else {
         EpiResidual<T> e{res, b, L.fixed, nullptr, nullptr};
@@ -1026,6 +1038,20 @@ void residual(tpo_problem *P, int li, const T *b, const T *x, T *res, const CGSt
     }
 }
 
+// The matrix of the coarsest level's sweeps for the current moduli.  Called before a V-cycle is
+// launched or captured: never inside a capture.
+void ensure_coarse_poly(tpo_problem *P) {
+    Level &C = P->L[P->nl - 1];
+    if (!C.S || C.S_version == P->E_version) return;
+    const int n = (int)C.g.ndof;
+    k_coarse_pack<<<nblk(81LL * n), 256, 0, P->s>>>(C.K, C.g, C.Sk);
+    CKL();
+    k_coarse_poly<<<nblk(n, 2), 1024, coarse_poly_smem(n), P->s>>>(C.Sk, C.g, C.invD, C.fixed, C.omega, C.womega,
+                                                                  P->mg.nu1 + P->mg.coarse_iters, C.S);
+    CKL();
+    C.S_version = P->E_version;
+}
+
 // x must be treated as zero on entry (it is fully overwritten).
 // rdot (level 0 only, may be null): fuse the PCG step r.z / beta into the last sweep of
 // an FP64 V-cycle; returns whether it did (not without a post-smoothing sweep).
@@ -1033,9 +1059,9 @@ template <typename T>
 bool vcycle(tpo_problem *P, int li, const T *b, T *x, const CGState *st, const double *rdot = nullptr) {
     Level &L = P->L[li];
     const bool last = li == P->nl - 1;
-    if (last && L.Kinv) {  // direct coarse solve: x = K^-1 b on the free DOFs
+    if (last && (L.Kinv || L.S)) {  // direct coarse solve (x = K^-1 b on the free DOFs) or the sweeps' matrix
         const int n = (int)L.g.ndof;
-        k_dense_mv<T><<<G(P, (n + 7) / 8), 256, 0, P->s>>>(L.Kinv, n, b, x, st);
+        k_dense_mv<T><<<G(P, (n + 7) / 8), 256, 0, P->s>>>(L.Kinv ? L.Kinv : L.S, n, b, x, st);
         CKL();
         return false;
     }
@@ -1047,8 +1073,15 @@ bool vcycle(tpo_problem *P, int li, const T *b, T *x, const CGState *st, const d
     int nsm = 0;       // sweeps done at this level
     int seq = 0;       // sweeps done in the current smoothing sequence (Chebyshev index)
     bool seq0 = true;  // the current sequence started from x = 0
+    // a dense level's first two sweeps are one launch
+    const bool first_two = L.dense && P->mg.nu1 >= 1 && P->mg.nu1 + (last ? P->mg.coarse_iters : 0) >= 2;
     auto do_smooth = [&]() {
-        if (nsm == 0) {
+        if (nsm == 0 && first_two) {
+            // left to the next call, which does both sweeps
+        } else if (nsm == 1 && first_two) {
+            smooth<T>(P, li, b, nullptr, alt, st, seq, seq0);
+            std::swap(cur, alt);
+        } else if (nsm == 0) {
             smooth_from_zero<T>(P, li, b, cur, st);
         } else {
             smooth<T>(P, li, b, cur, alt, st, seq, seq0);
@@ -1358,6 +1391,7 @@ void solve_fp64(tpo_problem *P, const tpo_solve_opts &o, tpo_solve_info *info) {
         P->use_tc_cg = false;
         P->tc_mode = o.tensor_cores >= 5 ? 2 : (o.tensor_cores >= 3 ? 1 : 0);
     }
+    if (o.precond == TPO_PREC_MG) ensure_coarse_poly(P);
     if (o.precond == TPO_PREC_BDDC) {
         if (P->nrhs > 1) fail(TPO_BAD_ARG, "the BDDC preconditioner solves one right-hand side at a time");
         if (P->bddc_iters != o.bddc_smoother_iters && P->gexec[kModeBddc]) {  // captured with another count
@@ -1421,6 +1455,7 @@ void solve_fp64(tpo_problem *P, const tpo_solve_opts &o, tpo_solve_info *info) {
 void solve_mixed(tpo_problem *P, const tpo_solve_opts &o, tpo_solve_info *info) {
     if (!P->have_E) fail(TPO_BAD_ARG, "tpo_solve: densities were never set");
     ensure_mixed(P);
+    ensure_coarse_poly(P);
     P->use_tc = o.tensor_cores >= 1;
     P->use_tc_cg = o.tensor_cores == 2 || o.tensor_cores == 4;
     P->tc_mode = o.tensor_cores >= 3 ? 1 : 0;
@@ -1876,6 +1911,7 @@ tpo_status tpo_vcycle(tpo_problem *p, const double *b, double *z) {
         if (!p || !b || !z) fail(TPO_BAD_ARG, "null argument");
         if (!p->have_E) fail(TPO_BAD_ARG, "densities were never set");
         const size_t nb = (size_t)p->g.ndof * sizeof(double);
+        ensure_coarse_poly(p);
         CK(cudaMemcpyAsync(p->r, b, nb, cudaMemcpyHostToDevice, p->s));
         vcycle<double>(p, 0, p->r, p->z, nullptr);
         CK(cudaMemcpyAsync(z, p->z, nb, cudaMemcpyDeviceToHost, p->s));

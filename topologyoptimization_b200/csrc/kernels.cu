@@ -116,28 +116,44 @@ __global__ void k_diag(const __grid_constant__ KeParam<double> ke, Grid g, const
 }
 
 // ---- dense Galerkin coarse levels (:628-699) --------------------------------------
-// Damping of the dense levels under safe_omega: damped Jacobi x += w D^-1 (b - K x)
-// converges (and keeps the symmetric V-cycle positive definite) iff w lambda_max(D^-1 K) < 2;
-// the Gershgorin row bound g >= lambda_max gives the damping w = min(omega, 1.9 / g).
-// Rows are summed in column order, as the oracle does.
-__global__ void k_dense_jacobi_bound(const double *__restrict__ K, int n, const uint8_t *__restrict__ fixed,
-                                     double omega, double *__restrict__ womega) {
-    double g = 0.0;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        const double d = K[(long long)i * n + i];
-        if (fixed[i] || !(d > 1e-30)) continue;
-        double s = 0.0;
-        for (int j = 0; j < n; j++) s += fabs(K[(long long)i * n + j]);
-        g = fmax(g, s / d);
+// Diagonal and damping of a dense level, one warp per row (_diagFromDense :742-751).  Under
+// safe_omega (womega not null) damped Jacobi x += w D^-1 (b - K x) converges (and keeps the
+// symmetric V-cycle positive definite) iff w lambda_max(D^-1 K) < 2; the Gershgorin row bound
+// g >= lambda_max gives w = min(omega, 1.9 / g).  womega[0] = w; the words behind it are the
+// maximum's bits (positive doubles order as their bits) and the count of finished blocks, both
+// zero between launches.  (One block that read the rows thread by thread took 1.0 ms at 1911
+// DOFs.)
+__global__ void k_dense_rows(const double *__restrict__ K, const Grid g, const uint8_t *__restrict__ fixed, double omega,
+                             double *__restrict__ invD, float *__restrict__ invD32, double *__restrict__ womega) {
+    const int n = (int)g.ndof, lane = threadIdx.x & 31;
+    const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    unsigned long long *bits = reinterpret_cast<unsigned long long *>(womega + 1);
+    unsigned long long *finished = reinterpret_cast<unsigned long long *>(womega + 2);
+    if (row < n) {
+        const double *Kr = K + (long long)row * n;
+        const double d = Kr[row];
+        const double v = (!fixed[row] && d > 1e-30) ? 1.0 / d : 0.0;
+        if (lane == 0) {
+            invD[row] = v;
+            invD32[row] = (float)v;
+        }
+        if (womega && v != 0.0) {
+            double s = 0.0;
+            for (int j = lane; j < n; j += 32) s += fabs(Kr[j]);
+            s = warp_sum(s);
+            if (lane == 0) atomicMax(bits, (unsigned long long)__double_as_longlong(s / d));
+        }
     }
-    for (int o = 16; o > 0; o >>= 1) g = fmax(g, __shfl_xor_sync(0xffffffffu, g, o));
-    __shared__ double sh[32];
-    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = g;
+    if (!womega) return;
     __syncthreads();
     if (threadIdx.x == 0) {
-        for (int w = 1; w < (int)(blockDim.x >> 5); w++) g = fmax(g, sh[w]);
-        g = fmax(g, sh[0]);
-        *womega = g > 0.0 ? fmin(omega, 1.9 / g) : omega;
+        __threadfence();
+        if (atomicAdd(finished, 1ULL) == gridDim.x - 1) {
+            __threadfence();
+            const double gb = __longlong_as_double((long long)atomicExch(bits, 0ULL));
+            womega[0] = gb > 0.0 ? fmin(omega, 1.9 / gb) : omega;
+            *finished = 0ULL;
+        }
     }
 }
 
@@ -252,17 +268,6 @@ __global__ void k_galerkin_PtT(Grid gf, Grid gc, const double *__restrict__ T, d
     Kc[t] = s;
 }
 
-// _diagFromDense (:742-751)
-__global__ void k_dense_invdiag(const double *__restrict__ K, int n, const uint8_t *__restrict__ fixed,
-                                double *__restrict__ invD, float *__restrict__ invD32) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const double d = K[(long long)i * n + i];
-    const double v = (!fixed[i] && d > 1e-30) ? 1.0 / d : 0.0;
-    invD[i] = v;
-    invD32[i] = (float)v;
-}
-
 // ---- coarsest level: explicit inverse of the dense operator -------------------------
 // The operator restricted to its free, non-singular DOFs: rows/columns whose inverse
 // diagonal is 0 (fixed DOFs, DOFs without active elements) become identity rows.
@@ -306,6 +311,91 @@ __global__ void k_coarse_mask_inverse(const double *__restrict__ Ainv, int n, co
     if (t >= (long long)n * n) return;
     const int i = (int)(t / n), j = (int)(t - (long long)i * n);
     Kinv[t] = (invD[i] == 0.0 || invD[j] == 0.0) ? 0.0 : Ainv[t];
+}
+
+// ---- coarsest level: its sweeps as one matrix -----------------------------------------
+// The reference solves the coarsest level by nu1 + 30 damped Jacobi sweeps from zero, a linear
+// map of b: x = S b.  S is formed once per hierarchy update, column by column (the sweeps on
+// b = e_c), and a V-cycle then needs one matrix-vector product there instead of 31 launches
+// (about 3 us each at 135 and 216 DOFs, half of a V-cycle's time on the worker's grids; S
+// itself takes 168 us at 216 DOFs).
+//
+// The operator's stencil entries, 81 a row (the order of dense_row_dot), 0 outside the grid.
+__global__ void k_coarse_pack(const double *__restrict__ K, const Grid g, double *__restrict__ Ks) {
+    const int n = (int)g.ndof, t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= 81 * n) return;
+    const int i = t / 81, e = t - 81 * i, line = e / 9, w = e - 9 * line;
+    int x, y, z;
+    node_xyz(g, i / 3, x, y, z);
+    const int xx = x + line / 3 - 1, yy = y + line % 3 - 1, zz = z + w / 3 - 1;
+    const bool in = xx >= 0 && xx < g.nnx && yy >= 0 && yy < g.nny && zz >= 0 && zz < g.nnz;
+    Ks[t] = in ? K[(long long)i * n + 3 * ((xx * g.nny + yy) * g.nnz + zz) + w % 3] : 0.0;
+}
+
+// A block runs `sweeps` sweeps on two columns held in shared memory (two copies, the columns
+// interleaved) with the table of the entries' columns; a warp takes a row at a time, three
+// entries a lane, and adds in the order of k_dense_smooth.  After the first exchange of the
+// reduction each half of the warp carries one column, so both sums cost one tree.  (One thread
+// per row, walking its 81 entries, took 376 us at 216 DOFs.)
+__global__ void __launch_bounds__(1024) k_coarse_poly(const double *__restrict__ Ks, const Grid g,
+                                                      const double *__restrict__ invD,
+                                                      const uint8_t *__restrict__ fixed, double omega,
+                                                      const double *__restrict__ womega, int sweeps,
+                                                      double *__restrict__ S) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int n = (int)g.ndof, c0 = blockIdx.x * 2;
+    double2 *cur = reinterpret_cast<double2 *>(smem_raw), *alt = cur + n;
+    unsigned short *col = reinterpret_cast<unsigned short *>(alt + n);
+    const double w = womega ? *womega : omega;
+    for (int t = threadIdx.x; t < 81 * n; t += blockDim.x) {
+        const int i = t / 81, e = t - 81 * i, line = e / 9, v = e - 9 * line;
+        int x, y, z;
+        node_xyz(g, i / 3, x, y, z);
+        const int xx = x + line / 3 - 1, yy = y + line % 3 - 1, zz = z + v / 3 - 1;
+        const bool in = xx >= 0 && xx < g.nnx && yy >= 0 && yy < g.nny && zz >= 0 && zz < g.nnz;
+        col[t] = in ? (unsigned short)(3 * ((xx * g.nny + yy) * g.nnz + zz) + v % 3) : (unsigned short)0;
+    }
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        const double d = fixed[i] ? 0.0 : w * invD[i];
+        cur[i] = make_double2(i == c0 ? d : 0.0, i == c0 + 1 ? d : 0.0);
+    }
+    const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    const bool upper = lane >= 16;
+    for (int k = 1; k < sweeps; k++) {
+        __syncthreads();
+        for (int i = threadIdx.x >> 5; i < n; i += nw) {
+            double s0 = 0.0, s1 = 0.0;
+#pragma unroll
+            for (int m = 0; m < 3; m++) {
+                const int e = lane + 32 * m;
+                if (e < 81) {
+                    const double kv = Ks[81 * i + e];
+                    const double2 xv = cur[col[81 * i + e]];
+                    s0 += kv * xv.x;
+                    s1 += kv * xv.y;
+                }
+            }
+            // lanes 0-15 go on with column 0, lanes 16-31 with column 1
+            const double give = upper ? s0 : s1;
+            double s = (upper ? s1 : s0) + __shfl_xor_sync(0xffffffffu, give, 16);
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+            if ((lane & 15) == 0) {
+                const int c = upper ? 1 : 0;
+                const double xi = reinterpret_cast<const double *>(cur)[2 * i + c];
+                const double bi = i == c0 + c ? 1.0 : 0.0;
+                reinterpret_cast<double *>(alt)[2 * i + c] = fixed[i] ? xi : xi + w * invD[i] * (bi - s);
+            }
+        }
+        double2 *t = cur;
+        cur = alt;
+        alt = t;
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        S[(long long)i * n + c0] = cur[i].x;
+        if (c0 + 1 < n) S[(long long)i * n + c0 + 1] = cur[i].y;
+    }
 }
 
 // ---- PCG (ebePCG assembly/index.ts:504-733, ebeMGPCG :1076-1193, FE :4189-4371) -----

@@ -36,14 +36,20 @@ __global__ void __launch_bounds__(128) k_galerkin_gather(const __grid_constant__
                                                          const double *__restrict__ EactF, double *__restrict__ Kc);
 __global__ void k_galerkin_T(Grid gf, Grid gc, const double *__restrict__ Kf, double *__restrict__ T);
 __global__ void k_galerkin_PtT(Grid gf, Grid gc, const double *__restrict__ T, double *__restrict__ Kc);
-__global__ void k_dense_invdiag(const double *__restrict__ K, int n, const uint8_t *__restrict__ fixed,
-                                double *__restrict__ invD, float *__restrict__ invD32);
-// Gershgorin bound g = max over free rows with a positive diagonal of sum_j |K_ij| / K_ii
-// (>= lambda_max(D^-1 K)); *womega = min(omega, 1.9 / g).  One block.
-__global__ void k_dense_jacobi_bound(const double *__restrict__ K, int n, const uint8_t *__restrict__ fixed,
-                                     double omega, double *__restrict__ womega);
+// womega: 3 doubles (damping, two words of scratch) or null
+__global__ void k_dense_rows(const double *__restrict__ K, const Grid g, const uint8_t *__restrict__ fixed, double omega,
+                             double *__restrict__ invD, float *__restrict__ invD32, double *__restrict__ womega);
 __global__ void k_dense_matvec_seq(const double *__restrict__ K, int n, const double *__restrict__ p,
                                    double *__restrict__ Ap);
+// coarsest level: its Jacobi sweeps from zero as a matrix
+constexpr int kPolyMaxN = 704;  // largest level that takes this form
+inline size_t coarse_poly_smem(int n) { return (size_t)n * (2 * sizeof(double2) + 81 * sizeof(unsigned short)); }
+__global__ void k_coarse_pack(const double *__restrict__ K, const Grid g, double *__restrict__ Ks);
+__global__ void __launch_bounds__(1024) k_coarse_poly(const double *__restrict__ Ks, const Grid g,
+                                                      const double *__restrict__ invD,
+                                                      const uint8_t *__restrict__ fixed, double omega,
+                                                      const double *__restrict__ womega, int sweeps,
+                                                      double *__restrict__ S);
 // coarsest level: explicit inverse
 __global__ void k_coarse_prepare(const double *__restrict__ K, int n, const double *__restrict__ invD,
                                  double *__restrict__ A);
