@@ -677,3 +677,50 @@ def test_vcycle_dense_levels(native, oracle, dims, kw):
     mg.update(1.0 - 0.5 * x, 2.0)
     assert rel_inf(z, zo) < 1e-11
     assert rel_inf(z2, mg.vcycle(b)) < 1e-11
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dims", [(1, 1, 1), (2, 7, 15), (3, 8, 16), (4, 9, 17), (30, 10, 10), (44, 44, 43), (44, 44, 44),
+                                  (70, 63, 60), (70, 63, 62)])
+def test_small_grid_apply(native, oracle, dims):
+    """The small-grid apply at its tile's edges (8 and 9 rows, 16 and 17 columns) and on both
+    sides of the rules' lines (90,000 and 280,000 nodes: one plane per block, two, the strip
+    kernel): K u with inactive elements and a spring, the FP32 apply, one V-cycle and a
+    batched solve.  Bounds of the suite's other applies: 1e-12 FP64, 2e-6 FP32."""
+    import torch
+    from topologyoptimization_b200 import Problem, mesh
+    from topologyoptimization_b200 import _native as N
+    rng = np.random.default_rng(12)
+    fixed = mesh.fixed_mask(*dims, "left")
+    x = rng.uniform(0.05, 1.0, int(np.prod(dims))).astype(np.float32)
+    x[rng.random(x.size) < 0.2] = 1e-3
+    u = rng.standard_normal(len(fixed))
+    E = 1e-9 + x.astype(np.float64) ** 3 * (1 - 1e-9)
+    act = np.flatnonzero(E > 1e-6).astype(np.int32)
+    ref = oracle.apply_a(oracle.lk(0.3), oracle.edofs3d(*dims), E, act, u)
+    dof = len(fixed) // 2
+    ref[dof] += 0.7 * u[dof]
+    with Problem(*dims, fixed) as P:
+        P.set_spring(dof, 0.7)
+        P.set_densities(x, 3.0)
+        assert rel_inf(P.apply(u), ref) < 1e-12
+        d_u, d_o = _dev(u.astype(np.float32)), torch.empty(len(u), dtype=torch.float32, device="cuda")
+        P.apply_f32_dev(d_u, d_o)
+        torch.cuda.synchronize()
+        assert rel_inf(d_o.cpu().numpy(), ref) < 2e-6
+        if min(dims) < 4:
+            return
+        P.set_spring(-1, 0.0)
+        b = u * (fixed == 0)
+        mg = oracle.MG(*dims, oracle.lk(0.3), fixed)
+        mg.update(x, 3.0)
+        assert rel_inf(P.vcycle(b), mg.vcycle(b)) < 1e-11
+        F = _dev(np.stack([b, 2.0 * b, b[::-1] * (fixed == 0)]))
+        U = torch.zeros_like(F)
+        o = N.default_solve_opts(max_iter=3, tol=0.0, ref_epsilon=0)
+        P.solve_multi_dev(F, U, o)
+        for k in range(3):
+            V = torch.zeros(len(u), dtype=torch.float64, device="cuda")
+            P.set_load(F[k])
+            P.solve_dev(V, o)
+            assert rel_inf(U[k].cpu().numpy(), V.cpu().numpy()) < 1e-10

@@ -19,6 +19,7 @@
 #include "../../include/tpo.h"
 #include "apply.cuh"
 #include "apply_tc.cuh"
+#include "apply_small.cuh"
 #include "apply_walsh.cuh"
 #include "kernels.cuh"
 #include "mg_kernels.cuh"
@@ -313,15 +314,57 @@ void configure_apply(size_t smem) {
             CK(cudaFuncSetAttribute(k_apply_w<T, Epi, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         apply_configured<T, Epi>() = smem;
     }
+    auto small = [](auto kernel, int tx) {
+        CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)small_smem<T>(tx)));
+    };
+    small(k_apply_small<T, Epi, false, 1>, 1);
+    small(k_apply_small<T, Epi, false, 2>, 2);
+    if constexpr (kDouble) {
+        small(k_apply_small<T, Epi, true, 1>, 1);
+        small(k_apply_small<T, Epi, true, 2>, 2);
+    }
     int per_sm = apply_per_sm<T, Epi, false>(smem);
     if constexpr (kDouble) per_sm = std::min(per_sm, apply_per_sm<T, Epi, true>(smem));
     const int conc = per_sm * (g_num_sms ? g_num_sms : 148);
     if (apply_conc<T, Epi>() == 0 || conc < apply_conc<T, Epi>()) apply_conc<T, Epi>() = conc;
 }
 
+// Node planes per CTA of the small-grid kernel, 0: the strip kernel.  Measured back to back in a
+// graph (us, FP64 / FP32; strip, one plane, two planes):
+//     16x8x8        1.4e3 nodes    5.7 / 6.2     3.1 / 2.8     3.8 / 3.3
+//     64x32x32      7.1e4          8.1 / 6.6     5.3 / 4.6     5.7 / 4.7
+//     75x37x39      1.2e5          9.9 / 8.5     8.8 / 6.8     9.6 / 5.8
+//     96x48x48      2.3e5         13.3 / 8.7    12.7 / 9.2    11.1 / 7.3
+//     110x52x58     3.5e5         15.2 / 10.6   21.4 / 14.1   18.9 / 11.9
+// The node count of a batched launch is that of all its right-hand sides.
+inline int small_planes(const Grid &g, int nrhs) {
+    const long long n = g.nnodes * nrhs;
+    if (g.nnx > 8192) return 0;  // blocks along x
+    return n <= 90000 ? 1 : (n <= 280000 ? 2 : 0);
+}
+template <typename T, class Epi, bool kGeneral>
+void launch_small(cudaStream_t st, const Grid &g, int tx, const WalshKe<T> &wk, const T *p, const T *Eact,
+                  const Epi &epi, const CGState *cg, int nrhs) {
+    const dim3 grid = small_grid(g, tx, (unsigned)nrhs);
+    const size_t smem = small_smem<T>(tx);
+    if (tx == 1) k_apply_small<T, Epi, kGeneral, 1><<<grid, kSThreads, smem, st>>>(wk, g, p, Eact, epi, cg);
+    else k_apply_small<T, Epi, kGeneral, 2><<<grid, kSThreads, smem, st>>>(wk, g, p, Eact, epi, cg);
+    CKL();
+}
+
 template <typename T, class Epi>
 void launch_apply(cudaStream_t st, const Grid &g, const WalshKe<T> &wk, const T *p, const T *Eact, const Epi &epi,
                   const CGState *cg, int nrhs = 1) {
+    if (const int tx = small_planes(g, nrhs)) {
+        if constexpr (std::is_same_v<T, double>) {
+            if (wk.general) {
+                launch_small<T, Epi, true>(st, g, tx, wk, p, Eact, epi, cg, nrhs);
+                return;
+            }
+        }
+        launch_small<T, Epi, false>(st, g, tx, wk, p, Eact, epi, cg, nrhs);
+        return;
+    }
     // the measured shape for launches without a grid-wide reduction (a reduction's order
     // follows the block count, which stays the cost model's so that results do not depend
     // on timing); batched launches keep the model, which counts their extra CTAs
@@ -968,7 +1011,7 @@ void tune_apply_shapes(tpo_problem *P) {
     if (cs != cudaStreamCaptureStatusNone) return;  // timing needs an uncaptured stream
     for (int li = 0; li < P->nl; li++) {
         Level &L = P->L[li];
-        if (L.dense) continue;
+        if (L.dense || small_planes(L.g, 1)) continue;
         tune_apply_shape<float>(P, L);
         tune_apply_shape<double>(P, L);
     }
@@ -1541,7 +1584,12 @@ tpo_problem *create_problem(const tpo_grid *gr, const double *Ke, double nu, con
         const long long tout = std::min(walsh_out_cols<double>(g.nnz), walsh_out_cols<float>(g.nnz));
         const long long tc_tiles = (long long)((g.nny + kTcNodesY - 1) / kTcNodesY) * ((g.nnz + kTcNodesZ - 1) / kTcNodesZ);
         const size_t colb = (size_t)std::max((ncol + tout - 1) / tout, tc_tiles);
-        P->npartials = 2 * std::max<size_t>(4096, colb * (size_t)std::min(g.nnx, 512));
+        size_t blocks = std::max<size_t>(4096, colb * (size_t)std::min(g.nnx, 512));
+        if (small_planes(g, 1)) {
+            const dim3 sg = small_grid(g, 1, 1);
+            blocks = std::max(blocks, (size_t)sg.x * sg.y);
+        }
+        P->npartials = 2 * blocks;
         P->partials = dalloc<double>(P->npartials);
         P->st = dalloc<CGState>(1);
         CK(cudaMemset(P->st, 0, sizeof(CGState)));
