@@ -122,3 +122,30 @@ def test_2d_bottom_support_side_load(native, oracle):
     assert r["iterations"] == ro["iterations"]
     assert first == n
     assert dc.max() < 1e-9
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dims", [(1, 1), (15, 15), (16, 15), (63, 31), (200, 60)])
+def test_2d_one_launch_solve(native, oracle, dims):
+    """The 2D worker's one-launch PCG with less than a block, exactly one block of 512 DOFs, one
+    row above it, eight full blocks and many: two SIMP iterations with inactive elements
+    against the oracle's loop.  Bounds of the suite's other short 2D runs: the same CG counts,
+    compliance 1e-7, x 1e-5."""
+    from topologyoptimization_b200 import mesh
+    from topologyoptimization_b200.worker2d import TopologyOptimizerWorker
+    nx, ny = dims
+    F = mesh.load_vector2d(nx, ny, "down")
+    fixed = mesh.fixed_mask2d(nx, ny, "left")
+    pres = np.zeros(nx * ny, np.uint8)
+    pres[mesh.constraint_elements2d(nx, ny, "left")] = 1
+    pres[mesh.force_elements2d(nx, ny, "down")] = 1
+    void = (np.random.default_rng(2).random(nx * ny) < 0.05).astype(np.uint8) * (1 - pres)
+    ro = oracle.simp2d(nx, ny, F, fixed, pres, void, max_iter=2, use_projection=1)
+    w = TopologyOptimizerWorker()
+    r = w.optimize({"nx": nx, "ny": ny}, dict(volumeFraction=0.3, maxIterations=2, penaltyFactor=3.0, filterRadius=1.5,
+                                              preservedElements=pres, voidElements=void))
+    n = min(ro["iterations"], r["iterations"])
+    assert np.array_equal(r["cgIterations"][:n], ro["cg"][:n])
+    assert np.abs(r["complianceHistory"][:n] / ro["compliance"][:n] - 1).max() < 1e-7
+    if ro["iterations"] == r["iterations"]:
+        assert np.abs(r["densities2D"] - ro["x"]).max() < 1e-5

@@ -150,3 +150,38 @@ def test_fe_pcg_warm_start(native, oracle, precond, dims):
     assert info.converged == 1 and ito < 5000
     assert rel_inf(Ug, Uo) < BAR
     assert _rel_c(info.compliance, F @ Uo) < BAR
+
+
+@pytest.mark.parametrize("dims,spring", [((1, 1, 1), False), ((3, 4, 5), True), ((30, 10, 10), True), ((16, 16, 16), False),
+                                         ((25, 19, 25), False), ((25, 27, 25), True), ((25, 34, 25), False), ((25, 41, 25), True),
+                                         ((25, 42, 25), False)])
+def test_jacobi_one_launch(native, oracle, dims, spring):
+    """The one-launch Jacobi-PCG at 1 to 6 nodes per lane (8 to 28,392 nodes, all but the largest
+    it takes) and just above (29,068, the graph of separate launches), with inactive elements and
+    a spring: the iterate after 10 iterations, warm start, against the oracle's recurrence
+    (before any of the grids has converged, where the recurrence divides rounding by rounding):
+    1e-10, as the other solves."""
+    from topologyoptimization_b200 import Problem
+    nel = int(np.prod(dims))
+    rng = np.random.default_rng(3)
+    x = rng.uniform(0.2, 1.0, nel).astype(np.float32)
+    if nel > 100:
+        x[rng.random(nel) < 0.1] = 1e-3
+    fixed = oracle.fixed_mask(*dims, "left")
+    F = cantilever_load(*dims) * SCALE
+    U0 = rng.standard_normal(len(F)) * (SCALE * 1e-3) * (fixed == 0)
+    mg = oracle.MG(*dims, oracle.lk(0.3), fixed)
+    dof = 3 * int((np.prod([d + 1 for d in dims])) - 1)
+    if spring:
+        mg.set_spring(dof, 0.4)
+    mg.update(x, 3.0)
+    n = min(10, int((fixed == 0).sum()) - 1)
+    Uo, ito = mg.fe_pcg(F, U0, n, 0.0, precond="jacobi")
+    with Problem(*dims, fixed) as P:
+        if spring:
+            P.set_spring(dof, 0.4)
+        P.set_densities(x, 3.0)
+        P.set_load(F)
+        Ug, info = P.solve(U0, precond=native.PREC_JACOBI, max_iter=n, tol=0.0, warm_start=1, ref_epsilon=1)
+    assert info.iterations == n and ito == n
+    assert rel_inf(Ug, Uo) < BAR

@@ -91,6 +91,8 @@ struct CGState {
     double rr32, maxr2, delta2;
     int do_update, n_updates;
     unsigned int counters[8];
+    unsigned int bar;  // arrivals at the grid barriers of a cooperative launch (zeroed before it)
+    int bar_err;       // one of its waits ran out
 };
 
 // Convergence decision after an iteration that produced ||r||^2 in st->rr, with the

@@ -1,6 +1,7 @@
 // Kernels whose arithmetic must follow the reference operation by operation.  This file
 // is compiled with --fmad=false so that a*b+c stays two rounded operations, as in
 // WebAssembly f64 and JavaScript.  Sums run in the reference's order.
+#include "cg_coop.cuh"
 #include "kernels.cuh"
 
 namespace tpo {
@@ -824,6 +825,137 @@ __global__ void k_evals_pow_f32(const float *__restrict__ x, int nel, double Emi
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= nel) return;
     E[e] = Emin + pow((double)x[e], penal) * (E0 - Emin);
+}
+
+// Jacobi-PCG of the 2D worker as one cooperative launch (cg_coop.cuh): one DOF per thread, its
+// four elements' products and their sum as k_csr_apply forms them, the vector updates and the
+// dot products as k_cg_alpha, k_cg_update_jacobi and k_cg_p do (their multiply-adds are fused,
+// and a block here is two of theirs: 256 DOFs a part), so the iterates are theirs bit for bit.
+__global__ void __launch_bounds__(kCoop2Threads) k_cg_coop2(const double *__restrict__ Ke, int nelx, int nely,
+                                                            const double *__restrict__ Em, double thresh,
+                                                            const double *__restrict__ invD,
+                                                            const uint8_t *__restrict__ fixed, double *U, double *r,
+                                                            double *z, double *pa, double *pb, CGState *st,
+                                                            double *parts) {
+    constexpr int NT = kCoop2Threads / 2, SEG = (NT + 2) * 2;
+    __shared__ double sp[3 * SEG], sK[64], sh[64], sh2[16];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int nny = nely + 1, ndof = 2 * (nelx + 1) * nny, nparts = (ndof + 255) / 256;
+    const int n0 = blockIdx.x * NT, d = 2 * n0 + tid, node = n0 + (tid >> 1), c = tid & 1;
+    if (tid < 64) sK[tid] = Ke[tid];
+    const bool own = d < ndof;
+    const int x = node / nny, y = node - x * nny;
+    // elements in ascending order; corner (ox, oy) of an element is its local node
+    // 0 (0,0), 1 (1,0), 2 (1,1), 3 (0,1)
+    double E[4];
+    bool have[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const int ex = x - 1 + (k >> 1), ey = y - 1 + (k & 1);
+        have[k] = own && ex >= 0 && ex < nelx && ey >= 0 && ey < nely;
+        E[k] = have[k] ? Em[ey + ex * nely] : 0.0;
+    }
+    const bool fx = own ? fixed[d] != 0 : true;
+    double Ud = own ? U[d] : 0.0, rd = own ? r[d] : 0.0;
+    const double dd = own ? invD[d] : 0.0;
+    const double eps = st->eps, tolSq = st->tolSq;
+    const int maxIter = st->maxIter;
+    CoopScalars s{st->rz, st->alpha, st->beta, st->rr, st->it, st->done};
+    const int it0 = s.it;
+    double *pold = pa, *pnew = pb;
+    unsigned epoch = 0;
+    bool ok = true;
+    // block sums of 256 threads each, as block_sum forms them
+    auto part_sums = [&](double a, double b, int nv, double *out) {
+        a = warp_sum(a);
+        if (nv == 2) b = warp_sum(b);
+        if (lane == 0) {
+            sh[warp] = a;
+            sh[32 + warp] = b;
+        }
+        __syncthreads();
+        if ((warp & 7) == 0) {
+            const int vb = 2 * blockIdx.x + (warp >> 3);
+            const double ta = warp_sum(lane < 8 ? sh[warp + lane] : 0.0);
+            const double tb = nv == 2 ? warp_sum(lane < 8 ? sh[32 + warp + lane] : 0.0) : 0.0;
+            if (lane == 0 && vb < nparts) {
+                out[vb] = ta;
+                if (nv == 2) out[nparts + vb] = tb;
+            }
+        }
+    };
+    while (!s.done && s.it - it0 < kCoopIters) {
+        constexpr int kLoads = (3 * SEG + kCoop2Threads - 1) / kCoop2Threads;
+        double zv[kLoads], pv[kLoads];
+#pragma unroll
+        for (int l = 0; l < kLoads; l++) {
+            const int i = l * kCoop2Threads + tid, sg = i / SEG, q = 2 * (n0 - 1 + (sg - 1) * nny) + (i - sg * SEG);
+            const bool in = i < 3 * SEG && q >= 0 && q < ndof;
+            zv[l] = in ? __ldcg(z + q) : 0.0;
+            pv[l] = in ? __ldcg(pold + q) : 0.0;
+        }
+#pragma unroll
+        for (int l = 0; l < kLoads; l++) {
+            const int i = l * kCoop2Threads + tid;
+            if (i < 3 * SEG) sp[i] = fma(s.beta, pv[l], zv[l]);
+        }
+        __syncthreads();
+        const double pd = sp[SEG + 2 + tid];
+        double ap = 0.0;
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const int ax = k >> 1, ay = k & 1;                                  // element (x-1+ax, y-1+ay)
+            const int i = 2 * (ay ? (ax ? 0 : 1) : (ax ? 3 : 2)) + c;           // this DOF in it
+            const double *col0 = sp + ax * SEG + 2 * ((tid >> 1) + ay), *col1 = col0 + SEG;  // nodes (ex, ey), (ex+1, ey)
+            if (have[k]) {
+                double yk = 0.0;
+                if (E[k] > thresh) {
+                    const double *Ki = sK + i * 8;
+                    double sum = 0.0;
+                    sum += Ki[0] * col0[0];
+                    sum += Ki[1] * col0[1];
+                    sum += Ki[2] * col1[0];
+                    sum += Ki[3] * col1[1];
+                    sum += Ki[4] * col1[2];
+                    sum += Ki[5] * col1[3];
+                    sum += Ki[6] * col0[2];
+                    sum += Ki[7] * col0[3];
+                    yk = E[k] * sum;
+                }
+                ap = ap + yk;
+            }
+        }
+        if (fx) ap = 0.0;
+        if (own) pnew[d] = pd;
+        part_sums(own ? pd * ap : 0.0, 0.0, 1, parts);
+        if (!(ok = grid_barrier(&st->bar, ++epoch * gridDim.x, &st->bar_err))) break;
+        double t1[1];
+        coop_total<1>(parts, nparts, sh2, t1);
+        if (!coop_alpha(s, t1[0], eps, st, blockIdx.x == 0 && tid == 0)) break;
+        rd = fma(-s.alpha, ap, rd);
+        const double zd = dd * rd;
+        Ud = fma(s.alpha, pd, Ud);
+        if (own) z[d] = zd;
+        part_sums(own ? rd * zd : 0.0, own ? rd * rd : 0.0, 2, parts + nparts);
+        if (!(ok = grid_barrier(&st->bar, ++epoch * gridDim.x, &st->bar_err))) break;
+        double t2[2];
+        coop_total<2>(parts + nparts, nparts, sh2, t2);
+        coop_beta(s, t2[0], t2[1], eps, tolSq, maxIter, st, blockIdx.x == 0 && tid == 0);
+        double *t = pold;
+        pold = pnew;
+        pnew = t;
+    }
+    if (own) {
+        U[d] = Ud;
+        r[d] = rd;
+    }
+    if (ok && blockIdx.x == 0 && tid == 0) {
+        st->rz = s.rz;
+        st->beta = s.beta;
+        st->rr = s.rr;
+        st->it = s.it;
+        st->done = s.done;
+    }
 }
 
 // _computeElementEnergyFlat (:335-345; js/optimizer-worker-3d.js:1561-1571): energy = sum_i

@@ -1,6 +1,7 @@
 // Multigrid transfers, diagonals, dense coarse levels, PCG vector kernels and the
 // element-energy kernel of libtpo.  Reference routines are cited per kernel
 // (Jozo132/TopologyOptimization paths).
+#include "cg_coop.cuh"
 #include "kernels.cuh"
 
 namespace tpo {

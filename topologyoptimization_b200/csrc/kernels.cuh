@@ -157,6 +157,13 @@ __global__ void k_filter_hs2d(int nelx, int nely, double rmin, float *__restrict
 __global__ void k_filter_sens2d(int nelx, int nely, double rmin, const float *__restrict__ Hs,
                                 const float *__restrict__ x, const float *__restrict__ dc, float *__restrict__ dcn);
 
+constexpr int kCoop2Threads = 512;
+__global__ void __launch_bounds__(kCoop2Threads) k_cg_coop2(const double *__restrict__ Ke, int nelx, int nely,
+                                                            const double *__restrict__ Em, double thresh,
+                                                            const double *__restrict__ invD,
+                                                            const uint8_t *__restrict__ fixed, double *U, double *r,
+                                                            double *z, double *pa, double *pb, CGState *st,
+                                                            double *parts);
 __global__ void k_cg_abs_tol(CGState *st, double tol);
 
 }  // namespace tpo
