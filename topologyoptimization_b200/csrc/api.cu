@@ -58,6 +58,33 @@ std::atomic<long long> g_launches{0};
         g_launches.fetch_add(1);      \
     } while (0)
 
+// A kernel of a solver iteration (one that begins with chain_sync): its launch may overlap the
+// end of the kernel before it in the stream.  It starts as soon as that one's blocks have all
+// started, and waits there for its results, so that a launch's 1 to 2 us of start-up is hidden.
+// Microseconds an iteration before -> after, with the FP32 / FP64 cycle: 94 / 97 -> 85 / 87 at
+// 32x16x16, 128 / 140 -> 120 / 132 at 64x32x32, 170 / 202 -> 167 / 200 at 96x48x48, 337 / 437
+// -> 327 / 428 at 150x74x78, 1057 / 1485 -> 1048 / 1478 at 256x128x128.
+struct Chain {
+    dim3 grid, block;
+    size_t smem;
+    cudaStream_t s;
+    template <typename... K, typename... A>
+    void operator()(void (*kernel)(K...), A &&...a) const {
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = grid;
+        cfg.blockDim = block;
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = s;
+        cudaLaunchAttribute at{};
+        at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at.val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = &at;
+        cfg.numAttrs = 1;
+        CK(cudaLaunchKernelEx(&cfg, kernel, K(a)...));
+        g_launches.fetch_add(1);
+    }
+};
+
 template <typename F>
 tpo_status guard(F &&f) {
     try {
@@ -108,6 +135,9 @@ void check_device() {
 
 inline unsigned nblk(long long n, int t = 256) { return (unsigned)std::max(1LL, (n + t - 1) / t); }
 inline unsigned red_blocks() { return (unsigned)std::max(1, (g_num_sms ? g_num_sms : 148) * 4); }
+// Blocks of a vector kernel on pairs of DOFs: one pair a thread up to red_blocks() (blocks without
+// work cost up to 1 us an iteration at 32x16x16).
+inline unsigned pair_blocks(long long n) { return std::min(red_blocks(), nblk((n + 1) / 2)); }
 
 KeParam<double> make_ke(const double *Ke) {
     KeParam<double> k;
@@ -346,11 +376,9 @@ inline int small_planes(const Grid &g, int nrhs) {
 template <typename T, class Epi, bool kGeneral>
 void launch_small(cudaStream_t st, const Grid &g, int tx, const WalshKe<T> &wk, const T *p, const T *Eact,
                   const Epi &epi, const CGState *cg, int nrhs) {
-    const dim3 grid = small_grid(g, tx, (unsigned)nrhs);
-    const size_t smem = small_smem<T>(tx);
-    if (tx == 1) k_apply_small<T, Epi, kGeneral, 1><<<grid, kSThreads, smem, st>>>(wk, g, p, Eact, epi, cg);
-    else k_apply_small<T, Epi, kGeneral, 2><<<grid, kSThreads, smem, st>>>(wk, g, p, Eact, epi, cg);
-    CKL();
+    const Chain launch{small_grid(g, tx, (unsigned)nrhs), dim3(kSThreads), small_smem<T>(tx), st};
+    if (tx == 1) launch(k_apply_small<T, Epi, kGeneral, 1>, wk, g, p, Eact, epi, cg);
+    else launch(k_apply_small<T, Epi, kGeneral, 2>, wk, g, p, Eact, epi, cg);
 }
 
 template <typename T, class Epi>
@@ -936,6 +964,11 @@ void build_hierarchy(tpo_problem *P, double Emin) {
 
 // Launch grid of a solve-path kernel: z = the right-hand sides of a batched solve.
 inline dim3 G(const tpo_problem *P, unsigned x) { return dim3(x, 1, (unsigned)P->nrhs); }
+// Whether a level's first sweep and its transfers are launched as Chain does.  With plain loads they
+// take longer where bandwidth counts (sweep, restriction, prolongation of 8 x 160x80x80: 49 -> 79,
+// 37 -> 40, 78 -> 110 us; of 256x128x128: 24 -> 25, -, 41 -> 44 us), more than a launch's start-up;
+// up to here they do not.
+inline bool chained(const tpo_problem *P, const Grid &g) { return g.ndof * P->nrhs <= 4000000; }
 
 // ---- precision-specific buffers ------------------------------------------------------
 template <typename T>
@@ -1027,9 +1060,14 @@ void smooth_from_zero(tpo_problem *P, int li, const T *b, T *x, const CGState *s
     Level &L = P->L[li];
     const long long nvec = (L.g.ndof + 15 / (long long)sizeof(T)) / (16 / (long long)sizeof(T));  // 16-byte vectors
     const T w = (T)(L.cheb ? L.cheb_w0 : L.omega);
-    k_smooth0<T><<<G(P, nblk(nvec)), 256, 0, P->s>>>(b, Prec<T>::invD(L), L.fixed, w, L.cheb ? nullptr : L.womega,
-                                                    x, L.g.ndof, st);
-    CKL();
+    if (chained(P, L.g)) {
+        Chain{G(P, nblk(nvec)), 256, 0, P->s}(k_smooth0<T, true>, b, Prec<T>::invD(L), L.fixed, w,
+                                              L.cheb ? nullptr : L.womega, x, L.g.ndof, st);
+    } else {
+        k_smooth0<T, false><<<G(P, nblk(nvec)), 256, 0, P->s>>>(b, Prec<T>::invD(L), L.fixed, w,
+                                                               L.cheb ? nullptr : L.womega, x, L.g.ndof, st);
+        CKL();
+    }
 }
 // Sweep number k (0-based) of a smoothing sequence from x into xn.  A Chebyshev level also
 // needs to know whether the sequence started at x = 0 (pre-smoothing).
@@ -1038,9 +1076,8 @@ void smooth(tpo_problem *P, int li, const T *b, const T *x, T *xn, const CGState
             bool from_zero = false) {
     Level &L = P->L[li];
     if (L.dense) {
-        k_dense_smooth<T><<<G(P, nblk(L.g.ndof, 8)), 256, 0, P->s>>>(L.K, L.g, x, b, Prec<T>::invD(L), L.fixed,
-                                                                    (T)L.omega, L.womega, xn, st);
-        CKL();
+        Chain{G(P, nblk(L.g.ndof, 8)), 256, 0, P->s}(k_dense_smooth<T>, L.K, L.g, x, b, Prec<T>::invD(L), L.fixed,
+                                                     (T)L.omega, L.womega, xn, st);
     } else if (L.cheb && k > 0) {
         if (k >= (int)L.cheb_cd.size()) fail(TPO_BAD_ARG, "Chebyshev sweep beyond the level's coefficients");
         EpiCheb<T> e{xn, b, Prec<T>::invD(L), L.fixed, (T)L.cheb_cd[k], (T)L.cheb_cr[k],
@@ -1068,8 +1105,7 @@ template <typename T>
 void residual(tpo_problem *P, int li, const T *b, const T *x, T *res, const CGState *st) {
     Level &L = P->L[li];
     if (L.dense) {
-        k_dense_residual<T><<<G(P, nblk(L.g.ndof, 8)), 256, 0, P->s>>>(L.K, L.g, x, b, L.fixed, res, st);
-        CKL();
+        Chain{G(P, nblk(L.g.ndof, 8)), 256, 0, P->s}(k_dense_residual<T>, L.K, L.g, x, b, L.fixed, res, st);
     } else {
         EpiResidual<T> e{res, b, L.fixed, nullptr, nullptr};
         if constexpr (std::is_same_v<T, float>) {
@@ -1105,8 +1141,7 @@ bool vcycle(tpo_problem *P, int li, const T *b, T *x, const CGState *st, const d
     const bool last = li == P->nl - 1;
     if (last && (L.Kinv || L.S)) {  // direct coarse solve (x = K^-1 b on the free DOFs) or the sweeps' matrix
         const int n = (int)L.g.ndof;
-        k_dense_mv<T><<<G(P, (n + 7) / 8), 256, 0, P->s>>>(L.Kinv ? L.Kinv : L.S, n, b, x, st);
-        CKL();
+        Chain{G(P, (n + 7) / 8), 256, 0, P->s}(k_dense_mv<T>, L.Kinv ? L.Kinv : L.S, n, b, x, st);
         return false;
     }
     // Every sweep after the first swaps the two buffers; start in whichever one makes the
@@ -1136,8 +1171,7 @@ bool vcycle(tpo_problem *P, int li, const T *b, T *x, const CGState *st, const d
     };
     for (int s = 0; s < P->mg.nu1; s++) do_smooth();
     if (nsm == 0) {
-        k_zero<T><<<G(P, nblk(L.g.ndof)), 256, 0, P->s>>>(cur, L.g.ndof, st);
-        CKL();
+        Chain{G(P, nblk(L.g.ndof)), 256, 0, P->s}(k_zero<T>, cur, L.g.ndof, st);
         nsm = 1;  // x is now an explicit zero; later sweeps need the operator
     }
     if (last) {
@@ -1146,11 +1180,23 @@ bool vcycle(tpo_problem *P, int li, const T *b, T *x, const CGState *st, const d
     } else {
         Level &C = P->L[li + 1];
         residual<T>(P, li, b, cur, Prec<T>::res(L), st);
-        k_restrict<T><<<restrict_grid(C.g, P->nrhs), restrict_block(C.g), 0, P->s>>>(L.g, C.g, Prec<T>::res(L), C.fixed, Prec<T>::b(C), st);
-        CKL();
+        if (chained(P, L.g)) {
+            Chain{restrict_grid(C.g, P->nrhs), restrict_block(C.g), 0, P->s}(
+                k_restrict<T, true>, L.g, C.g, Prec<T>::res(L), C.fixed, Prec<T>::b(C), st);
+        } else {
+            k_restrict<T, false><<<restrict_grid(C.g, P->nrhs), restrict_block(C.g), 0, P->s>>>(
+                L.g, C.g, Prec<T>::res(L), C.fixed, Prec<T>::b(C), st);
+            CKL();
+        }
         vcycle<T>(P, li + 1, Prec<T>::b(C), Prec<T>::x(C), st);
-        k_prolong<T><<<prolong_grid<T>(L.g, P->nrhs), prolong_block<T>(L.g), 0, P->s>>>(L.g, C.g, Prec<T>::x(C), L.fixed, cur, st);
-        CKL();
+        if (chained(P, L.g)) {
+            Chain{prolong_grid<T>(L.g, P->nrhs), prolong_block<T>(L.g), 0, P->s}(
+                k_prolong<T, true>, L.g, C.g, Prec<T>::x(C), L.fixed, cur, st);
+        } else {
+            k_prolong<T, false><<<prolong_grid<T>(L.g, P->nrhs), prolong_block<T>(L.g), 0, P->s>>>(
+                L.g, C.g, Prec<T>::x(C), L.fixed, cur, st);
+            CKL();
+        }
         seq = 0;  // post-smoothing: a new sequence from the prolonged iterate
         seq0 = false;
         // FP64 only: in the FP32 apply the epilogue's FP64 operands spill registers and the
@@ -1170,14 +1216,12 @@ bool vcycle(tpo_problem *P, int li, const T *b, T *x, const CGState *st, const d
             }
         }
         if (cur != x) {
-            k_copy<T><<<G(P, nblk(L.g.ndof)), 256, 0, P->s>>>(cur, x, L.g.ndof, st);
-            CKL();
+            Chain{G(P, nblk(L.g.ndof)), 256, 0, P->s}(k_copy<T>, cur, x, L.g.ndof, st);
         }
         return fuse;
     }
     if (cur != x) {
-        k_copy<T><<<G(P, nblk(L.g.ndof)), 256, 0, P->s>>>(cur, x, L.g.ndof, st);
-        CKL();
+        Chain{G(P, nblk(L.g.ndof)), 256, 0, P->s}(k_copy<T>, cur, x, L.g.ndof, st);
     }
     return false;
 }
@@ -1287,8 +1331,7 @@ void bddc_apply(tpo_problem *P, const double *r, double *z, const CGState *st) {
     const long long n = L0.g.ndof;
     const int napply = std::max(P->bddc_iters, 1);
     double *cur = (napply & 1) ? L0.xt : z, *alt = (napply & 1) ? z : L0.xt;
-    k_bddc_local<<<G(P, red_blocks()), 256, 0, P->s>>>(P->bddc_S, P->bddc_W, r, cur, n, st);
-    CKL();
+    Chain{G(P, red_blocks()), 256, 0, P->s}(k_bddc_local, P->bddc_S, P->bddc_W, r, cur, n, st);
     for (int k = 1; k < napply; k++) {
         EpiSmooth<double> e{alt, r, L0.invD, L0.fixed, 1.0, nullptr, nullptr};
         launch_apply<double>(P->s, L0.g, P->wk, cur, L0.Eact, e, st, P->nrhs);
@@ -1311,13 +1354,10 @@ void enqueue_iteration(tpo_problem *P, int mode) {
     if (f32_precond) {
         EpiCG<double> e{P->Ap, L0.fixed, P->st, P->partials, &P->st->counters[5]};
         launch_apply<double>(P->s, L0.g, P->wk, P->p, L0.Eact, e, P->st, P->nrhs);
-        k_cgP_update<<<G(P, red_blocks()), 256, 0, P->s>>>(P->U, P->r, P->r32, P->p, P->Ap, n, P->st, P->partials);
-        CKL();
+        Chain{G(P, pair_blocks(n)), 256, 0, P->s}(k_cgP_update, P->U, P->r, P->r32, P->p, P->Ap, n, P->st, P->partials);
         vcycle<float>(P, 0, P->r32, P->z32, P->st);
-        k_cgP_rz<<<G(P, red_blocks()), 256, 0, P->s>>>(P->r, P->z32, L0.fixed, n, P->st, P->partials);
-        CKL();
-        k_cgP_p<<<G(P, red_blocks()), 256, 0, P->s>>>(P->p, P->z32, n, P->st);
-        CKL();
+        Chain{G(P, pair_blocks(n)), 256, 0, P->s}(k_cgP_rz, P->r, P->z32, L0.fixed, n, P->st, P->partials);
+        Chain{G(P, pair_blocks(n)), 256, 0, P->s}(k_cgP_p, P->p, P->z32, n, P->st);
         return;
     }
     if (fp32_recurrence) {
@@ -1338,25 +1378,19 @@ void enqueue_iteration(tpo_problem *P, int mode) {
     EpiCG<double> e{P->Ap, L0.fixed, P->st, P->partials, &P->st->counters[5]};
     launch_apply<double>(P->s, L0.g, P->wk, P->p, L0.Eact, e, P->st, P->nrhs);
     if (mode == 0) {
-        k_cg_update_mg<<<G(P, red_blocks()), 256, 0, P->s>>>(P->U, P->r, P->p, P->Ap, n, P->st, P->partials);
-        CKL();
+        Chain{G(P, pair_blocks(n)), 256, 0, P->s}(k_cg_update_mg, P->U, P->r, P->p, P->Ap, n, P->st, P->partials);
         if (!vcycle<double>(P, 0, P->r, P->z, P->st, P->r)) {
-            k_cg_rz<<<G(P, red_blocks()), 256, 0, P->s>>>(P->r, P->z, L0.fixed, n, P->st, P->partials);
-            CKL();
+            Chain{G(P, pair_blocks(n)), 256, 0, P->s}(k_cg_rz, P->r, P->z, L0.fixed, n, P->st, P->partials);
         }
     } else if (mode == kModeBddc) {
-        k_cg_update_mg<<<G(P, red_blocks()), 256, 0, P->s>>>(P->U, P->r, P->p, P->Ap, n, P->st, P->partials);
-        CKL();
+        Chain{G(P, pair_blocks(n)), 256, 0, P->s}(k_cg_update_mg, P->U, P->r, P->p, P->Ap, n, P->st, P->partials);
         bddc_apply(P, P->r, P->z, P->st);
-        k_cg_rz<<<G(P, red_blocks()), 256, 0, P->s>>>(P->r, P->z, L0.fixed, n, P->st, P->partials);
-        CKL();
+        Chain{G(P, pair_blocks(n)), 256, 0, P->s}(k_cg_rz, P->r, P->z, L0.fixed, n, P->st, P->partials);
     } else {
-        k_cg_update_jacobi<<<G(P, red_blocks()), 256, 0, P->s>>>(P->U, P->r, P->z, P->p, P->Ap, L0.invD, n, P->st,
-                                                             P->partials);
-        CKL();
+        Chain{G(P, red_blocks()), 256, 0, P->s}(k_cg_update_jacobi, P->U, P->r, P->z, P->p, P->Ap, L0.invD, n, P->st,
+                                               P->partials);
     }
-    k_cg_p<<<G(P, red_blocks()), 256, 0, P->s>>>(P->p, P->z, n, P->st);
-    CKL();
+    Chain{G(P, pair_blocks(n)), 256, 0, P->s}(k_cg_p, P->p, P->z, n, P->st);
 }
 
 cudaGraphExec_t get_iteration_graph(tpo_problem *P, int mode, int chunk) {

@@ -128,8 +128,9 @@ inline dim3 small_grid(const Grid &g, int tx, unsigned nrhs) {
 
 template <typename T, class Epi, bool kGeneral, int TX>
 __global__ void __launch_bounds__(kSThreads)
-k_apply_small(const __grid_constant__ WalshKe<T> wk, const Grid g, const T *__restrict__ p, const T *__restrict__ Eact,
-              Epi epi, const CGState *__restrict__ st) {
+k_apply_small(const __grid_constant__ WalshKe<T> wk, const Grid g, const T *p, const T *Eact, Epi epi,
+              const CGState *st) {
+    chain_sync();
     using S = SmallV<T>;
     using V = typename S::V;
     if (blockIdx.z) {  // right-hand side of a batched solve
@@ -159,7 +160,7 @@ k_apply_small(const __grid_constant__ WalshKe<T> wk, const Grid g, const T *__re
 #pragma unroll
         for (int i0 = 0; i0 < kSPlane; i0 += kSThreads) {
             const int i = i0 + tid, r = i / kSPitch, c = i - r * kSPitch;
-            if (i < kSPlane) slab[x * kSPlane + i] = in && r < srows && c < scols ? __ldg(src + x * plane3 + r * row3 + c) : T(0);
+            if (i < kSPlane) slab[x * kSPlane + i] = in && r < srows && c < scols ? src[x * plane3 + r * row3 + c] : T(0);
         }
     }
     // this thread's element column and its moduli, planes x0 - 1 .. x0 + TX - 1
@@ -169,7 +170,7 @@ k_apply_small(const __grid_constant__ WalshKe<T> wk, const Grid g, const T *__re
     T E[TX + 1];
 #pragma unroll
     for (int x = 0; x < TX + 1; x++)
-        E[x] = eok && (unsigned)(x0 - 1 + x) < (unsigned)g.nelx ? __ldg(ep + (long long)x * g.nely * g.nelz) : T(0);
+        E[x] = eok && (unsigned)(x0 - 1 + x) < (unsigned)g.nelx ? ep[(long long)x * g.nely * g.nelz] : T(0);
     // the node this thread finishes: column `col` of every plane
     const bool nok = tid < kSCols && yb + eb < g.nny && zb + ez < nnz && (eb > 0 || yti == 0) && (ez > 0 || zti == 0);
     const long long dof = x0 * plane3 + (long long)(yb + eb) * row3 + 3 * (zb + ez);

@@ -152,6 +152,22 @@ __device__ __forceinline__ void st_pair(T *a, long long i, Pair<T> v, bool vec) 
     }
 }
 
+// Start of every kernel of a solver iteration.  Under a programmatic launch (Chain of api.cu) the
+// kernel may have started while the one before it still ran: wait for that one's memory, then
+// let the next one start in turn.  Without that launch attribute both are no-ops.  What such a
+// kernel reads may change while it waits here, so its inputs are plain pointers: __restrict__
+// const or __ldg would let the compiler take them for constant over the whole launch.
+__device__ __forceinline__ void chain_sync() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+// An input of a kernel that is launched both ways: the read-only path where no launch overlaps.
+template <bool kChain, typename T>
+__device__ __forceinline__ T ld_in(const T *p) {
+    if constexpr (kChain) return *p;
+    else return __ldg(p);
+}
+
 // ---- reductions --------------------------------------------------------------
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll

@@ -497,8 +497,9 @@ __global__ void k_cg_pz(const double *__restrict__ r, double *__restrict__ z, co
 }
 
 // U += alpha p; r -= alpha Ap; rr = r.r (MG variant: z comes from the V-cycle next).
-__global__ void k_cg_update_mg(double *__restrict__ U, double *__restrict__ r, const double *__restrict__ p,
-                               const double *__restrict__ Ap, long long n, CGState *st, double *partials) {
+__global__ void k_cg_update_mg(double *U, double *r, const double *p, const double *Ap, long long n, CGState *st,
+                               double *partials) {
+    chain_sync();
     const long long zr = blockIdx.z;  // right-hand side of a batched solve (0 otherwise)
     U += zr * n;
     r += zr * n;
@@ -538,8 +539,9 @@ __global__ void k_cg_update_mg(double *__restrict__ U, double *__restrict__ r, c
 }
 
 // z zeroed on fixed DOFs; rz_new = r.z; beta.
-__global__ void k_cg_rz(const double *__restrict__ r, double *__restrict__ z, const uint8_t *__restrict__ fixed,
-                        long long n, CGState *st, double *partials) {
+__global__ void k_cg_rz(const double *r, double *z, const uint8_t *fixed, long long n, CGState *st,
+                        double *partials) {
+    chain_sync();
     const long long zr = blockIdx.z;  // right-hand side of a batched solve (0 otherwise)
     r += zr * n;
     z += zr * n;
@@ -580,9 +582,9 @@ __global__ void k_cg_rz(const double *__restrict__ r, double *__restrict__ z, co
 }
 
 // Jacobi variant: U += alpha p; r -= alpha Ap; z = invD r; rz_new and rr in one pass.
-__global__ void k_cg_update_jacobi(double *__restrict__ U, double *__restrict__ r, double *__restrict__ z,
-                                   const double *__restrict__ p, const double *__restrict__ Ap,
-                                   const double *__restrict__ invD, long long n, CGState *st, double *partials) {
+__global__ void k_cg_update_jacobi(double *U, double *r, double *z, const double *p, const double *Ap,
+                                   const double *invD, long long n, CGState *st, double *partials) {
+    chain_sync();
     if (st->done) return;
     const double alpha = st->alpha;
     double v[2] = {0.0, 0.0};
@@ -607,7 +609,8 @@ __global__ void k_cg_update_jacobi(double *__restrict__ U, double *__restrict__ 
     }
 }
 
-__global__ void k_cg_p(double *__restrict__ p, const double *__restrict__ z, long long n, const CGState *st) {
+__global__ void k_cg_p(double *p, const double *z, long long n, const CGState *st) {
+    chain_sync();
     const long long zr = blockIdx.z;  // right-hand side of a batched solve (0 otherwise)
     p += zr * n;
     z += zr * n;
@@ -894,9 +897,9 @@ __global__ void k_bddc_setup(const __grid_constant__ KeParam<double> ke, Grid g,
 }
 
 // z = S r / W (grid z: right-hand sides)
-__global__ void k_bddc_local(const double *__restrict__ S, const uint8_t *__restrict__ W,
-                             const double *__restrict__ r, double *__restrict__ z, long long n,
-                             const CGState *__restrict__ st) {
+__global__ void k_bddc_local(const double *S, const uint8_t *W, const double *r, double *z, long long n,
+                             const CGState *st) {
+    chain_sync();
     if (blockIdx.z) {
         r += blockIdx.z * n;
         z += blockIdx.z * n;

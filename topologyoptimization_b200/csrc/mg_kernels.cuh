@@ -35,9 +35,9 @@ dim3 prolong_block(const Grid &gf) {
 // weights are powers of two, so the result equals the reference's scatter loop bit for
 // bit.  Each fine z-plane's 27 values are loaded unconditionally (indices outside the grid
 // clamped to its edge, their terms then skipped), so they are in flight together.
-template <typename T>
-__global__ void k_restrict(Grid gf, Grid gc, const T *__restrict__ res, const uint8_t *__restrict__ fixedC,
-                           T *__restrict__ bC, const CGState *st) {
+template <typename T, bool kChain>
+__global__ void k_restrict(Grid gf, Grid gc, const T *res, const uint8_t *fixedC, T *bC, const CGState *st) {
+    if constexpr (kChain) chain_sync();
     const long long zr = blockIdx.z;  // right-hand side of a batched solve (0 otherwise)
     res += zr * gf.ndof;
     bC += zr * gc.ndof;
@@ -86,7 +86,7 @@ __global__ void k_restrict(Grid gf, Grid gc, const T *__restrict__ res, const ui
 #pragma unroll
             for (int ix = 0; ix < 3; ix++)
 #pragma unroll
-                for (int d = 0; d < 3; d++) v[iy][ix][d] = __ldg(row[ix][iy] + 3 * fz[iz] + d);
+                for (int d = 0; d < 3; d++) v[iy][ix][d] = ld_in<kChain>(row[ix][iy] + 3 * fz[iz] + d);
 #pragma unroll
         for (int iy = 0; iy < 3; iy++)
 #pragma unroll
@@ -109,9 +109,9 @@ __global__ void k_restrict(Grid gf, Grid gc, const T *__restrict__ res, const ui
 // 000,100,...,111, so it rounds exactly as the full 8-term sum with its zero terms.  The
 // corner values, x and the mask are loaded unconditionally (a missing corner reads c0
 // again), so the loads are in flight together.
-template <typename T>
-__global__ void k_prolong(Grid gf, Grid gc, const T *__restrict__ xC, const uint8_t *__restrict__ fixedF,
-                          T *__restrict__ x, const CGState *st) {
+template <typename T, bool kChain>
+__global__ void k_prolong(Grid gf, Grid gc, const T *xC, const uint8_t *fixedF, T *x, const CGState *st) {
+    if constexpr (kChain) chain_sync();
     const long long zr = blockIdx.z;  // right-hand side of a batched solve (0 otherwise)
     xC += zr * gc.ndof;
     x += zr * gf.ndof;
@@ -145,7 +145,7 @@ __global__ void k_prolong(Grid gf, Grid gc, const T *__restrict__ xC, const uint
     T xq[3];
 #pragma unroll
     for (int d = 0; d < 3; d++) {
-        fm[d] = fixedF[q + d];
+        fm[d] = ld_in<kChain>(fixedF + q + d);
         xq[d] = x[q + d];
     }
     T c[8][3];
@@ -153,7 +153,7 @@ __global__ void k_prolong(Grid gf, Grid gc, const T *__restrict__ xC, const uint
     for (int k = 0; k < 8; k++)
 #pragma unroll
         for (int d = 0; d < 3; d++)
-            c[k][d] = __ldg(c00 + ((k & 1) ? ox : 0) + ((k & 2) ? oy : 0) + ((k & 4) ? oz : 0) + d);
+            c[k][d] = ld_in<kChain>(c00 + ((k & 1) ? ox : 0) + ((k & 2) ? oy : 0) + ((k & 4) ? oz : 0) + d);
 #pragma unroll
     for (int d = 0; d < 3; d++) {
         T val = c[0][d] * w;
@@ -170,7 +170,7 @@ __global__ void k_prolong(Grid gf, Grid gc, const T *__restrict__ xC, const uint
 // the 27-point stencil of its node, nine runs of nine columns (z - 1 .. z + 1 of the lines
 // (x + dx, y + dy)), three entries a lane.  xf(j) is the vector.  Sum in every lane.
 template <class F>
-__device__ __forceinline__ double dense_row_dot(const Grid &g, const double *__restrict__ Kr, int row, int lane, F xf) {
+__device__ __forceinline__ double dense_row_dot(const Grid &g, const double *Kr, int row, int lane, F xf) {
     const int node = row / 3, r = node / g.nnz;
     const int z = node - r * g.nnz, x = r / g.nny, y = r - x * g.nny;
     double s = 0.0;
@@ -190,9 +190,9 @@ __device__ __forceinline__ double dense_row_dot(const Grid &g, const double *__r
 // the first two sweeps of a sequence from zero in one pass, x_j = w D^-1 b there.
 // (Reading the whole row took 16 us a sweep at 1911 DOFs, 4.7 us at 675.)
 template <typename T>
-__global__ void k_dense_smooth(const double *__restrict__ K, const Grid g, const T *__restrict__ x,
-                               const T *__restrict__ b, const T *__restrict__ invD, const uint8_t *__restrict__ fixed,
-                               T omega, const double *__restrict__ womega, T *__restrict__ xn, const CGState *st) {
+__global__ void k_dense_smooth(const double *K, const Grid g, const T *x, const T *b, const T *invD,
+                               const uint8_t *fixed, T omega, const double *womega, T *xn, const CGState *st) {
+    chain_sync();
     const int n = (int)g.ndof;
     const long long zr = blockIdx.z;  // right-hand side of a batched solve (0 otherwise)
     if (x) x += zr * n;
@@ -213,9 +213,9 @@ __global__ void k_dense_smooth(const double *__restrict__ K, const Grid g, const
     }
 }
 template <typename T>
-__global__ void k_dense_residual(const double *__restrict__ K, const Grid g, const T *__restrict__ x,
-                                 const T *__restrict__ b, const uint8_t *__restrict__ fixed, T *__restrict__ res,
-                                 const CGState *st) {
+__global__ void k_dense_residual(const double *K, const Grid g, const T *x, const T *b, const uint8_t *fixed,
+                                 T *res, const CGState *st) {
+    chain_sync();
     const int n = (int)g.ndof;
     const long long zr = blockIdx.z;  // right-hand side of a batched solve (0 otherwise)
     x += zr * n;
@@ -233,6 +233,7 @@ __global__ void k_dense_residual(const double *__restrict__ K, const Grid g, con
 // ---- vectors ------------------------------------------------------------------------
 template <typename T>
 __global__ void k_zero(T *a, long long n, const CGState *st) {
+    chain_sync();
     const long long zr = blockIdx.z;  // right-hand side of a batched solve (0 otherwise)
     a += zr * n;
     if (st) st += zr;
@@ -241,7 +242,8 @@ __global__ void k_zero(T *a, long long n, const CGState *st) {
         a[i] = T(0);
 }
 template <typename T>
-__global__ void k_copy(const T *__restrict__ a, T *__restrict__ b, long long n, const CGState *st) {
+__global__ void k_copy(const T *a, T *b, long long n, const CGState *st) {
+    chain_sync();
     const long long zr = blockIdx.z;  // right-hand side of a batched solve (0 otherwise)
     a += zr * n;
     b += zr * n;
@@ -251,10 +253,10 @@ __global__ void k_copy(const T *__restrict__ a, T *__restrict__ b, long long n, 
         b[i] = a[i];
 }
 // First smoothing sweep from x = 0: x = 0 + omega*invD*(b - A*0), so no operator apply.
-template <typename T>
-__global__ void k_smooth0(const T *__restrict__ b, const T *__restrict__ invD, const uint8_t *__restrict__ fixed,
-                          T omega, const double *__restrict__ womega, T *__restrict__ x, long long n,
-                          const CGState *st) {
+template <typename T, bool kChain>
+__global__ void k_smooth0(const T *b, const T *invD, const uint8_t *fixed, T omega, const double *womega, T *x,
+                          long long n, const CGState *st) {
+    if constexpr (kChain) chain_sync();
     const long long zr = blockIdx.z;  // right-hand side of a batched solve (0 otherwise)
     b += zr * n;
     x += zr * n;
@@ -272,9 +274,9 @@ __global__ void k_smooth0(const T *__restrict__ b, const T *__restrict__ invD, c
     const long long nv = vec_ok ? n / V : 0;
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nv; i += stride) {
-        const Vec bv = reinterpret_cast<const Vec *>(b)[i];
-        const Vec dv = reinterpret_cast<const Vec *>(invD)[i];
-        const Fx fv = reinterpret_cast<const Fx *>(fixed)[i];
+        const Vec bv = ld_in<kChain>(reinterpret_cast<const Vec *>(b) + i);
+        const Vec dv = ld_in<kChain>(reinterpret_cast<const Vec *>(invD) + i);
+        const Fx fv = ld_in<kChain>(reinterpret_cast<const Fx *>(fixed) + i);
         const T *bs = reinterpret_cast<const T *>(&bv);
         const T *ds = reinterpret_cast<const T *>(&dv);
         const unsigned char *fs = reinterpret_cast<const unsigned char *>(&fv);
@@ -284,8 +286,10 @@ __global__ void k_smooth0(const T *__restrict__ b, const T *__restrict__ invD, c
         for (int j = 0; j < V; j++) xs[j] = fs[j] ? T(0) : T(0) + w * ds[j] * bs[j];
         reinterpret_cast<Vec *>(x)[i] = xv;
     }
-    for (long long i = nv * V + blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += stride)
-        x[i] = fixed[i] ? T(0) : T(0) + w * invD[i] * b[i];
+    for (long long i = nv * V + blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += stride) {
+        const T bv = ld_in<kChain>(b + i), dv = ld_in<kChain>(invD + i);
+        x[i] = ld_in<kChain>(fixed + i) ? T(0) : T(0) + w * dv * bv;
+    }
 }
 
 // ---- PCG on T-precision vectors with FP64 scalars (inner solve of the mixed-precision
@@ -492,9 +496,9 @@ __global__ void k_cgP_pz(const double *__restrict__ r, float *__restrict__ z32, 
 }
 
 // U += alpha p; r -= alpha Ap (FP64); r32 = (float) r; ||r||^2; convergence decision.
-__global__ void k_cgP_update(double *__restrict__ U, double *__restrict__ r, float *__restrict__ r32,
-                             const double *__restrict__ p, const double *__restrict__ Ap, long long n, CGState *st,
-                             double *partials) {
+__global__ void k_cgP_update(double *U, double *r, float *r32, const double *p, const double *Ap, long long n,
+                             CGState *st, double *partials) {
+    chain_sync();
     const long long zr = blockIdx.z;  // right-hand side of a batched solve (0 otherwise)
     U += zr * n;
     r += zr * n;
@@ -537,8 +541,9 @@ __global__ void k_cgP_update(double *__restrict__ U, double *__restrict__ r, flo
 }
 
 // z32 zeroed on fixed DOFs; rz_new = r.z32 (FP64); beta.
-__global__ void k_cgP_rz(const double *__restrict__ r, float *__restrict__ z32, const uint8_t *__restrict__ fixed,
-                         long long n, CGState *st, double *partials) {
+__global__ void k_cgP_rz(const double *r, float *z32, const uint8_t *fixed, long long n, CGState *st,
+                         double *partials) {
+    chain_sync();
     const long long zr = blockIdx.z;  // right-hand side of a batched solve (0 otherwise)
     r += zr * n;
     z32 += zr * n;
@@ -579,7 +584,8 @@ __global__ void k_cgP_rz(const double *__restrict__ r, float *__restrict__ z32, 
 }
 
 // p = z32 + beta p (FP64 direction).
-__global__ void k_cgP_p(double *__restrict__ p, const float *__restrict__ z32, long long n, const CGState *st) {
+__global__ void k_cgP_p(double *p, const float *z32, long long n, const CGState *st) {
+    chain_sync();
     const long long zr = blockIdx.z;  // right-hand side of a batched solve (0 otherwise)
     p += zr * n;
     z32 += zr * n;
@@ -602,8 +608,8 @@ __global__ void k_cgP_p(double *__restrict__ p, const float *__restrict__ z32, l
 // x = M b on the coarsest level (M: the inverse of its operator, or its sweeps as a matrix),
 // one warp per row.
 template <typename T>
-__global__ void k_dense_mv(const double *__restrict__ K, int n, const T *__restrict__ b, T *__restrict__ x,
-                           const CGState *st) {
+__global__ void k_dense_mv(const double *K, int n, const T *b, T *x, const CGState *st) {
+    chain_sync();
     const long long zr = blockIdx.z;  // right-hand side of a batched solve (0 otherwise)
     b += zr * n;
     x += zr * n;
