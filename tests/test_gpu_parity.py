@@ -680,6 +680,27 @@ def test_vcycle_dense_levels(native, oracle, dims, kw):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("island", [False, True])
+@pytest.mark.parametrize("dims", [(4, 4, 4), (6, 6, 6), (12, 4, 4), (6, 6, 8), (24, 6, 10), (30, 10, 10)])
+def test_coarse_inverse_edges(native, oracle, dims, island):
+    """The coarsest operator's inverse at the edges of its pivot blocks (32) and tiles (64): 81,
+    192, 189, 240, 936 and 1728 DOFs, with and without a part of the structure that floats
+    (its pivots vanish and are replaced).  Within the other direct V-cycles' 1e-9."""
+    from topologyoptimization_b200 import Problem, mesh
+    fixed = mesh.fixed_mask(*dims, "left")
+    x = _densities(int(np.prod(dims)), 51, 0.3, 1.0)
+    if island:
+        h, w = dims[0] // 2, 2 if dims[0] >= 12 else 0  # a void of four elements cuts the coarse grid too
+        x.reshape(dims[2], dims[1], dims[0])[:, :, h - w:h + w] = 1e-3
+    b = np.random.default_rng(52).standard_normal(len(fixed)) * (fixed == 0)
+    mg = oracle.MG(*dims, oracle.lk(0.3), fixed, coarse_direct=1, max_levels=2)
+    mg.update(x, 3.0)
+    with Problem(*dims, fixed, mg=native.default_mg_opts(coarse_direct=1, max_levels=2)) as P:
+        P.set_densities(x, 3.0)
+        assert rel_inf(P.vcycle(b), mg.vcycle(b)) < 1e-9
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("dims", [(1, 1, 1), (2, 7, 15), (3, 8, 16), (4, 9, 17), (30, 10, 10), (44, 44, 43), (44, 44, 44),
                                   (70, 63, 60), (70, 63, 62)])
 def test_small_grid_apply(native, oracle, dims):

@@ -281,28 +281,120 @@ __global__ void k_coarse_prepare(const double *__restrict__ K, int n, const doub
     A[t] = (ci || cj) ? (i == j ? 1.0 : 0.0) : K[t];
 }
 
-// One Gauss-Jordan sweep of pivot k, A -> B (both n x n, row-major): after sweeping every
-// pivot of a symmetric positive definite A in turn, the matrix holds A^-1.  The pivot
+// Gauss-Jordan sweeps of the pivots k0 .. k0 + 31, A -> B (both n x n, row-major): after sweeping
+// every pivot of a symmetric positive definite A in turn, the matrix holds A^-1.  The pivot
 // a_kk at step k is the Schur complement of the pivots swept before it, i.e. the d of a
 // Cholesky factorisation; a pivot at or below 1e-10 of the row's diagonal (1 / invD, or 1
 // on a decoupled row) is a singular direction up to rounding (a floating island of active
 // elements) and is replaced by 1, the same modification of A as the oracle's Cholesky
-// makes.  Reading A and writing B keeps the pivot row and column intact while they are read.
-__global__ void k_gj_sweep(const double *__restrict__ A, double *__restrict__ B, int n, int k,
-                           const double *__restrict__ invD) {
-    const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (t >= (long long)n * n) return;
-    const int i = (int)(t / n), j = (int)(t - (long long)i * n);
-    const double dk = invD[k] == 0.0 ? 1.0 : 1.0 / invD[k];
-    double p = A[(long long)k * n + k];
-    if (!(p > 1e-10 * dk)) p = 1.0;
-    const double ip = 1.0 / p;
-    const double aik = A[(long long)i * n + k], akj = A[(long long)k * n + j];
-    double v;
-    if (i == k) v = (j == k) ? ip : akj * ip;
-    else if (j == k) v = -aik * ip;
-    else v = A[t] - aik * (akj * ip);
-    B[t] = v;
+// makes.
+//
+// With K the block's pivots and D = A_KK, sweeping them in turn gives B_KK = D^-1, B_Kj =
+// D^-1 A_Kj, B_iK = -A_iK D^-1 and B_ij = A_ij - A_iK D^-1 A_Kj: every CTA sweeps D for itself
+// in shared memory (a chain of 32 divisions and barriers, which bounds the launch) while its
+// 64 x 64 tile and the two panels are on their way, and then takes the tile through the block
+// with one read and one write.  One launch per pivot instead moved the matrix 32 times as often
+// and was bound by launches: a hierarchy update with 135, 336, 675 coarsest DOFs took 0.54,
+// 1.12, 3.26 ms and takes 0.30, 0.48, 0.77.
+__global__ void __launch_bounds__(kGjThreads) k_gj_block(const double *__restrict__ A, double *__restrict__ B, int n,
+                                                         int k0, const double *__restrict__ invD) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    double *d0 = reinterpret_cast<double *>(smem_raw), *d1 = d0 + kGjNb * kGjPitch;  // D between two steps
+    double *ai = d1 + kGjNb * kGjPitch;   // A_iK, 64 x 32
+    double *ak = ai + kGjTile * kGjPitch; // A_Kj, 32 x 64
+    double *y = ak + kGjNb * kGjTile;     // D^-1 A_Kj; D^-1 in the columns of K
+    double *least = y + kGjNb * kGjTile;
+    const int tid = threadIdx.x, nb = min(kGjNb, n - k0);
+    const int i0 = blockIdx.y * kGjTile, j0 = blockIdx.x * kGjTile;
+    const int tx = tid & 15, ty = tid >> 4;
+    double a[4][4];  // rows ty + 16 r, columns tx + 16 c of the tile; 0 in the columns of K
+#pragma unroll
+    for (int r = 0; r < 4; r++)
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+            const int i = i0 + ty + 16 * r, j = j0 + tx + 16 * c;
+            a[r][c] = i < n && j < n && (j < k0 || j >= k0 + nb) ? A[(long long)i * n + j] : 0.0;
+        }
+    for (int t = tid; t < kGjNb * kGjNb; t += kGjThreads) {
+        const int r = t / kGjNb, c = t - r * kGjNb;
+        d0[r * kGjPitch + c] = r < nb && c < nb ? A[(long long)(k0 + r) * n + k0 + c] : 0.0;
+    }
+    if (tid < nb) {
+        const double di = invD[k0 + tid];
+        least[tid] = 1e-10 * (di == 0.0 ? 1.0 : 1.0 / di);
+    }
+    for (int t = tid; t < kGjTile * kGjNb; t += kGjThreads) {
+        const int r = t / kGjNb, c = t - r * kGjNb;
+        ai[r * kGjPitch + c] = i0 + r < n && c < nb ? A[(long long)(i0 + r) * n + k0 + c] : 0.0;
+        const int kr = t / kGjTile, kc = t - kr * kGjTile;
+        ak[t] = kr < nb && j0 + kc < n ? A[(long long)(k0 + kr) * n + j0 + kc] : 0.0;
+    }
+    __syncthreads();
+
+    // D <- D^-1, one pivot after the other
+    const int dc = tid & 31, dr = tid >> 5;
+    for (int k = 0; k < nb; k++) {
+        double p = d0[k * kGjPitch + k];
+        if (!(p > least[k])) p = 1.0;
+        const double ip = 1.0 / p;
+        const double s = d0[k * kGjPitch + dc] * ip;
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const int r = dr + 8 * q;
+            const double arc = d0[r * kGjPitch + dc], ark = d0[r * kGjPitch + k];
+            double v;
+            if (r == k) v = dc == k ? ip : s;
+            else if (dc == k) v = -ark * ip;
+            else v = arc - ark * s;
+            d1[r * kGjPitch + dc] = v;
+        }
+        double *t = d0;
+        d0 = d1;
+        d1 = t;
+        __syncthreads();
+    }
+
+    // y: rows ty and ty + 16, four columns
+    {
+        double v[2][4] = {};
+#pragma unroll 8
+        for (int k = 0; k < kGjNb; k++) {
+            const double l0 = d0[ty * kGjPitch + k], l1 = d0[(ty + 16) * kGjPitch + k];
+#pragma unroll
+            for (int c = 0; c < 4; c++) {
+                const double b = ak[k * kGjTile + tx + 16 * c];
+                v[0][c] += l0 * b;
+                v[1][c] += l1 * b;
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < 2; r++)
+#pragma unroll
+            for (int c = 0; c < 4; c++) {
+                const int row = ty + 16 * r, kj = j0 + tx + 16 * c - k0;
+                y[row * kGjTile + tx + 16 * c] = kj >= 0 && kj < nb ? d0[row * kGjPitch + kj] : v[r][c];
+            }
+    }
+    __syncthreads();
+#pragma unroll 4
+    for (int k = 0; k < kGjNb; k++) {
+        double l[4], b[4];
+#pragma unroll
+        for (int r = 0; r < 4; r++) l[r] = ai[(ty + 16 * r) * kGjPitch + k];
+#pragma unroll
+        for (int c = 0; c < 4; c++) b[c] = y[k * kGjTile + tx + 16 * c];
+#pragma unroll
+        for (int r = 0; r < 4; r++)
+#pragma unroll
+            for (int c = 0; c < 4; c++) a[r][c] -= l[r] * b[c];
+    }
+#pragma unroll
+    for (int r = 0; r < 4; r++)
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+            const int i = i0 + ty + 16 * r, j = j0 + tx + 16 * c, ki = i - k0;
+            if (i < n && j < n) B[(long long)i * n + j] = ki >= 0 && ki < nb ? y[ki * kGjTile + tx + 16 * c] : a[r][c];
+        }
 }
 
 // Kinv = Ainv with zero rows and columns on DOFs whose invD is 0 (their coarse solution is 0).

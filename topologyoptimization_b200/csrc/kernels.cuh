@@ -53,7 +53,10 @@ __global__ void __launch_bounds__(1024) k_coarse_poly(const double *__restrict__
 // coarsest level: explicit inverse
 __global__ void k_coarse_prepare(const double *__restrict__ K, int n, const double *__restrict__ invD,
                                  double *__restrict__ A);
-__global__ void k_gj_sweep(const double *__restrict__ A, double *__restrict__ B, int n, int k,
+constexpr int kGjNb = 32, kGjTile = 64, kGjThreads = 256;  // pivots a launch, tile of a CTA
+constexpr int kGjPitch = kGjNb + 1;
+constexpr size_t kGjSmem = sizeof(double) * (2 * kGjNb * kGjPitch + kGjTile * kGjPitch + 2 * kGjNb * kGjTile + kGjNb);
+__global__ void k_gj_block(const double *__restrict__ A, double *__restrict__ B, int n, int k0,
                            const double *__restrict__ invD);
 __global__ void k_coarse_mask_inverse(const double *__restrict__ Ainv, int n, const double *__restrict__ invD,
                                       double *__restrict__ Kinv);
