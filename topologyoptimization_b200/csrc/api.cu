@@ -1720,7 +1720,6 @@ void ensure_simp_arrays(tpo_problem *P) {
 struct OcCtx {
     cudaStream_t s;
     OCState *oc, *oc_host;
-    double *partials;
     long long n;
 };
 
@@ -1737,14 +1736,13 @@ void run_oc_ctx(const OcCtx &c, const float *d_x, double volfrac, const float *d
     long long per = (c.n + blocks - 1) / blocks;
     if (per >= (1LL << 31)) fail(TPO_BAD_ARG, "too many elements for the OC update");
     const size_t room = (size_t)std::max(optin - 8 * 1024, 0);  // beside the kernel's static arrays
-    int cap = (int)std::min<long long>(per, (long long)(room / sizeof(float2)));
-    const size_t smem = (size_t)cap * sizeof(float2);
+    int cap = (int)std::min<long long>(per, (long long)(room / kOcElemBytes));
+    const size_t smem = (size_t)cap * kOcElemBytes;
     CK(cudaFuncSetAttribute(k_oc_bisect, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)room));
     CK(cudaMemsetAsync(c.oc, 0, sizeof(OCState), c.s));
     long long n = c.n;
     OCState *oc = c.oc;
-    unsigned long long *words = reinterpret_cast<unsigned long long *>(c.partials);
-    void *args[] = {&d_x, &d_dc, &pres, &voidm, &n, &per, &cap, &volfrac, &move, &max_bisections, &oc, &words, &d_xold, &d_xnew};
+    void *args[] = {&d_x, &d_dc, &pres, &voidm, &n, &per, &cap, &volfrac, &move, &max_bisections, &oc, &d_xold, &d_xnew};
     CK(cudaLaunchCooperativeKernel((const void *)k_oc_bisect, dim3((unsigned)blocks), dim3(kOcThreads), args, smem, c.s));
     CKL();
     CK(cudaMemcpyAsync(c.oc_host, c.oc, sizeof(OCState), cudaMemcpyDeviceToHost, c.s));
@@ -1762,7 +1760,7 @@ void run_oc_ctx(const OcCtx &c, const float *d_x, double volfrac, const float *d
 void run_oc(tpo_problem *P, const float *d_x, double volfrac, const float *d_dc, const uint8_t *pres,
             const uint8_t *voidm, float *d_xnew, const float *d_xold, double *lmid, int *nb, double *change,
             double move = 0.2, int max_bisections = 1280) {
-    const OcCtx c{P->s, P->oc, P->oc_host, P->partials, P->g.nel};
+    const OcCtx c{P->s, P->oc, P->oc_host, P->g.nel};
     run_oc_ctx(c, d_x, volfrac, d_dc, pres, voidm, d_xnew, d_xold, lmid, nb, change, move, max_bisections);
 }
 
@@ -3014,7 +3012,7 @@ tpo_status tpo_simp2d_step_dev(tpo_problem2d *p, const tpo_simp2d_opts *o, float
         CK(cudaStreamSynchronize(s));
         const double compliance = p->scal_host[0];
         double change = 0.0;
-        const OcCtx c{s, p->oc, p->oc_host, p->partials, ne};
+        const OcCtx c{s, p->oc, p->oc_host, ne};
         run_oc_ctx(c, p->xold, o->volfrac, p->dcn, d_preserved, d_void, d_x, p->xold, nullptr, nullptr, &change, 0.2,
                    1280);
         if (info) {

@@ -491,14 +491,19 @@ __device__ double x192_to_double(const Exact192 &a) {
 }
 
 // ---- the whole bisection in one cooperative launch ---------------------------------------
-// A value's sum in units of 2^-51: v in [2^-28, 2) is a multiple of 2^-51, and the bits of
-// v + 2.0 minus those of 2.0 are v 2^51 (same binade, no rounding).  2^51 times 4096 values
-// below 2 stays inside 64 bits.
+// Values a thread adds before its 64-bit sums go to the 192-bit one: 4096 below 2 in units of
+// 2^-51 (below 2^-28 in units of 2^-79) stay inside 64 bits.
 constexpr int kFastFlush = 4096;
 
 __device__ __forceinline__ void x192_add_u51(Exact192 &a, unsigned long long u) {
     // u 2^-51 = u 2^98 2^-149: limb 1, offset 34
     const Exact192 t{0ULL, u << 34, u >> 30, 0u};
+    x192_add(a, t);
+}
+
+__device__ __forceinline__ void x192_add_u79(Exact192 &a, unsigned long long u) {
+    // u 2^-79 = u 2^70 2^-149: limb 1, offset 6
+    const Exact192 t{0ULL, u << 6, u >> 58, 0u};
     x192_add(a, t);
 }
 
@@ -523,111 +528,175 @@ __device__ __forceinline__ Exact192 x192_block_sum(Exact192 acc, Exact192 *sh) {
     return acc;
 }
 
-// xnew(lmid) of one element as oc_xnew forms it.  rl = 1 / lmid in FP32: an FP32 estimate of
-// s = x sqrt(-dc / lmid) (relative error below 1e-6 in the range tested) decides an element
-// that lies clear of the move limits, where the result is the limit itself; the others, and
-// every value outside the estimate's range (NaN included), take the FP64 division and root.
-__device__ __forceinline__ float oc_xnew_fast(float xf, float dcf, double lmid, float rl, double move) {
+// One element of the bisection.  xnew(lmid) rounds max(0, max(lo, min(1, min(hi, s)))) to FP32, with
+// lo, hi = x -+ move and s = x sqrt(-dc / lmid).  Rounding is monotone, so it is the same to
+// clamp (float)s by (float)lo and (float)hi, and lmid only enters s = t / sqrt(lmid), t = x
+// sqrt(-dc): one FP64 product a step instead of a division and a root.
+struct __align__(16) OcElem {
+    double t;      // NaN: take oc_xnew
+    int lo, hi;    // bits of max(0, (float)lo) and min(1, (float)hi); floats >= 0 order as integers
+};
+static_assert(sizeof(OcElem) == kOcElemBytes, "shared-memory size of an element");
+__device__ __forceinline__ OcElem oc_elem(float xf, float dcf, double move) {
     const double x = (double)xf, lo = x - move, hi = x + move;
-    const float bf = -dcf * rl;
-    if (bf < 1e30f) {
-        const float sf = xf * sqrtf(bf);
-        const float hf = fminf((float)hi, 1.0f), lf = (float)lo;
-        if (sf > hf * 1.00001f && sf < 1e30f && hf > 1e-6f) return (float)js_max(0.0, js_max(lo, js_min(1.0, hi)));
-        if (sf < lf * 0.99999f && lf > 1e-6f) return (float)js_max(0.0, js_max(lo, js_min(1.0, lo)));
-    }
-    return oc_xnew(xf, dcf, nullptr, nullptr, 0, lmid, move);
+    OcElem e;
+    e.t = lo == lo && hi == hi ? x * sqrt(-(double)dcf) + 0.0 : __longlong_as_double(0x7ff8000000000000LL);
+    e.lo = max(0, __float_as_int((float)lo));
+    e.hi = min(0x3f800000, __float_as_int((float)hi));
+    return e;
+}
+// The bits of xnew, or -1 where the product does not decide.  s' = t rl, rl = lmid^-1/2, is within
+// 8 units of the last place of the reference's FP64 s (each takes at most four roundings), so
+// both round to the same float unless s' lies within 16 units of a midpoint of two floats
+// (6e-8 of all values).  NaN, negative values and those too small to round here are not
+// decided either; from 2^30 on min(1, hi) decides.
+__device__ __forceinline__ int oc_bits(const OcElem &e, double rl) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(e.t * rl);
+    const unsigned h = (unsigned)(b >> 32), low = (unsigned)b & 0x1fffffffu;
+    const bool in = h >= 0x38700000u && h < 0x7ff00000u && low - (0x10000000u - 16u) > 32u;
+    int f = (int)((unsigned)((b + 0x10000000ULL) >> 29) - (896u << 23));  // nearest float
+    f = h >= 0x41d00000u ? 0x4e800000 : f;
+    f = b == 0 ? 0 : f;
+    return in || b == 0 ? max(e.lo, min(e.hi, f)) : -1;
 }
 
 // OC (js/optimizer-worker-3d.js:3066-3101): bisection on the multiplier, then xnew at the last
 // one and change = max |xnew - xold|.  Block b owns elements [b per, (b + 1) per); it keeps the
-// first `cap` of them (x, dc) in shared memory for all steps.  Each step every block sums its
-// xnew exactly, publishes the four words, passes the grid barrier and adds up all blocks'
-// words itself (integers: the same total everywhere), so a step costs one barrier.  Preserved
-// and void elements contribute a constant, added once.  partials: 2 x 4 words per block.
+// first `cap` of them in shared memory for all steps.  Each step every block sums its xnew
+// exactly and adds the sum to the step's words (integers: the total does not depend on the
+// order), and after the grid barrier every block reads the total and takes the same step.
+// Preserved and void elements contribute a constant, added once.
 //
-// One launch per step, each with its last block adding the partials of 592 blocks in one
-// thread, took 47-54 us a step whatever the size (24,000 to 2,000,000 elements): the serial
-// sum.  Here a step is bound by the barrier (about 2.5 us) up to 100,000 elements and by the
-// per-element arithmetic beyond.
+// A value in [2^-28, 2) is a multiple of 2^-51 and adds to one 64-bit sum, one in [2^-56, 2^-28) a
+// multiple of 2^-79 to another; what else there is goes through the 192-bit sum.
+//
+// One launch per step took 47-54 us a step whatever the size.  In this launch a step is bound by
+// its barrier and two block reductions (3 to 4 us) up to 200,000 elements and by 25 instructions
+// an element beyond.  With a division and a root for every warp that holds an element between
+// its limits, and every block adding up all blocks' words, a call of nine steps took 74, 112,
+// 210, 347 us for 24,000, 524,288, 2.05M and 4.2M elements; it takes 67, 80, 118, 234 (the last
+// keeps only half of its elements in shared memory).
 __global__ void __launch_bounds__(kOcThreads) k_oc_bisect(const float *x, const float *dc,
                                                           const uint8_t *__restrict__ pres,
                                                           const uint8_t *__restrict__ voidm, long long n, long long per,
                                                           int cap, double volfrac, double move, int max_bisections,
-                                                          OCState *s, unsigned long long *partials, const float *xold,
-                                                          float *xnew) {
+                                                          OCState *s, const float *xold, float *xnew) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    float2 *sv = reinterpret_cast<float2 *>(smem_raw);
+    OcElem *sv = reinterpret_cast<OcElem *>(smem_raw);
     __shared__ Exact192 sh[32];
-    __shared__ double s_l[3];
+    __shared__ unsigned piece[4][32];
+    __shared__ double s_l[4];
     __shared__ int s_done;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const long long b0 = blockIdx.x * per, b1 = min(n, b0 + per);
     const int ne = (int)max(0LL, b1 - b0);
     const int ns = min(ne, cap);
-    Exact192 base{0ULL, 0ULL, 0ULL, 0u};  // preserved elements: 1 each
-    // masked elements enter the loop as x = dc = 0, whose xnew is 0
-    auto load = [&](int i) {
+    auto elem = [&](int i) {
         const long long e = b0 + i;
-        return (pres && pres[e]) || (voidm && voidm[e]) ? make_float2(0.f, 0.f) : make_float2(x[e], dc[e]);
+        if (pres && pres[e]) return OcElem{0.0, 0x3f800000, 0x3f800000};  // 1
+        if (voidm && voidm[e]) return OcElem{0.0, 0, 0};
+        return oc_elem(x[e], dc[e], move);
     };
-    for (int i = threadIdx.x; i < ne; i += blockDim.x)
-        if (pres && pres[b0 + i]) x192_add_u51(base, 1ULL << 51);
-    for (int i = threadIdx.x; i < ns; i += blockDim.x) sv[i] = load(i);
-    __syncthreads();
-    double l1 = 0.0, l2 = 1e9, lmid = 0.0, sum = 0.0;
+    for (int i = threadIdx.x; i < ns; i += blockDim.x) sv[i] = elem(i);
+    double l1 = 0.0, l2 = 1e9, lmid = 0.0, rl = 0.0, sum = 0.0;
+    auto value = [&](int i) {  // bits of xnew(lmid)
+        int r = oc_bits(i < ns ? sv[i] : elem(i), rl);
+        if (r < 0) r = __float_as_int(oc_xnew(x[b0 + i], dc[b0 + i], nullptr, nullptr, 0, lmid, move));
+        return r;
+    };
+    // lmid^-1/2; NaN, which decides no element, for multipliers near the end of the range
+    auto root = [](double l) { return l > 1e-290 ? rsqrt(l) : __longlong_as_double(0x7ff8000000000000LL); };
     int nb = 0;
     bool done = !((l2 - l1) / (l2 + l1) > 1e-3);
+    double lnext = 0.5 * (l2 + l1), rnext = root(lnext);
     while (!done && nb < max_bisections) {
-        lmid = 0.5 * (l2 + l1);
-        const float rl = (float)(1.0 / lmid);
-        Exact192 acc = base;
-        unsigned long long fast = 0ULL;
+        lmid = lnext;
+        rl = rnext;
+        Exact192 acc{0ULL, 0ULL, 0ULL, 0u};
+        unsigned long long fast = 0ULL, tiny = 0ULL;
+        bool rare = false;
         int nf = 0;
-        auto add = [&](float2 v) {
-            const float r = oc_xnew_fast(v.x, v.y, lmid, rl, move);
-            if (r >= 0x1p-28f && r < 2.0f) {
-                fast += (unsigned long long)(__double_as_longlong((double)r + 2.0) - 0x4000000000000000LL);
-                if (++nf == kFastFlush) {
-                    x192_add_u51(acc, fast);
-                    fast = 0ULL;
-                    nf = 0;
-                }
-            } else if (r != 0.0f) {
-                x192_add_float(acc, r);
+        for (int i = threadIdx.x; i < ne; i += blockDim.x) {
+            const int r = value(i);
+            const unsigned e = (unsigned)r >> 23;
+            const unsigned long long m = ((unsigned)r & 0x7fffffu) | 0x800000u;
+            if (e - 99u < 29u) {
+                fast += m << (e - 99u);
+            } else if (e - 71u < 28u) {
+                tiny += m << (e - 71u);
+            } else if (r != 0) {
+                x192_add_float(acc, __int_as_float(r));
+                rare = true;
             }
-        };
-        for (int i = threadIdx.x; i < ns; i += blockDim.x) add(sv[i]);
-        for (int i = ns + threadIdx.x; i < ne; i += blockDim.x) add(load(i));
-        x192_add_u51(acc, fast);
-        __syncthreads();  // sh is free (the previous step's readers are past it)
-        acc = x192_block_sum(acc, sh);
-        unsigned long long *pw = partials + (size_t)(nb & 1) * 4 * gridDim.x;
-        if (threadIdx.x == 0) {
-            pw[4 * blockIdx.x + 0] = acc.w0;
-            pw[4 * blockIdx.x + 1] = acc.w1;
-            pw[4 * blockIdx.x + 2] = acc.w2;
-            pw[4 * blockIdx.x + 3] = acc.nan;
+            if (++nf == kFastFlush) {
+                x192_add_u51(acc, fast);
+                x192_add_u79(acc, tiny);
+                fast = tiny = 0ULL;
+                rare = true;
+                nf = 0;
+            }
+        }
+        OcWords *w = &s->words[nb % 3];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {  // 16 bits of every thread's sum at a time
+            const unsigned p = __reduce_add_sync(0xffffffffu, (unsigned)(fast >> (16 * k)) & 0xffffu);
+            if (lane == 0) piece[k][wid] = p;
+        }
+        if (__syncthreads_or(rare || tiny != 0ULL)) {
+            x192_add_u79(acc, tiny);
+            acc = x192_block_sum(acc, sh);
+            if (threadIdx.x == 0) {
+                const unsigned long long l[3] = {acc.w0, acc.w1, acc.w2};
+                for (int k = 0; k < 3; k++) {
+                    if (!l[k]) continue;
+                    atomicAdd(&w->limb[2 * k], l[k] & 0xffffffffULL);
+                    atomicAdd(&w->limb[2 * k + 1], l[k] >> 32);
+                }
+                if (acc.nan) atomicAdd(&w->nan, 1ULL);
+            }
+        }
+        if (wid < 4) {
+            const unsigned p = __reduce_add_sync(0xffffffffu, lane < (int)(blockDim.x >> 5) ? piece[wid][lane] : 0u);
+            if (lane == 0 && p) atomicAdd(&w->piece[wid], (unsigned long long)p);
         }
         if (!grid_barrier(&s->bar, (unsigned)(nb + 1) * gridDim.x, &s->err)) return;
-        if (threadIdx.x < 32) {
-            Exact192 tot{0ULL, 0ULL, 0ULL, 0u};
-            for (unsigned b = threadIdx.x; b < gridDim.x; b += 32) {
-                const Exact192 pb{__ldcg(&pw[4 * b + 0]), __ldcg(&pw[4 * b + 1]), __ldcg(&pw[4 * b + 2]),
-                                  (unsigned int)__ldcg(&pw[4 * b + 3])};
-                x192_add(tot, pb);
-            }
+        // the words of the step before are read everywhere: clear them for the step after the next
+        if (blockIdx.x == 0 && wid == 1 && lane < kOcWords)
+            reinterpret_cast<unsigned long long *>(&s->words[(nb + 2) % 3])[lane] = 0ULL;
+        if (wid == 0) {
+            const unsigned long long v =
+                lane < kOcWords ? __ldcg(reinterpret_cast<unsigned long long *>(w) + lane) : 0ULL;
+            const bool limbs = __any_sync(0xffffffffu, lane >= 4 && v != 0ULL);
+            unsigned long long p[4];
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                const Exact192 b = x192_shfl_down(tot, o);
-                x192_add(tot, b);
+            for (int k = 0; k < 4; k++) p[k] = __shfl_sync(0xffffffffu, v, k);
+            Exact192 tot{0ULL, 0ULL, (p[2] + (p[3] << 16)) << 2, 0u};  // 2^-19 = 2^130 2^-149
+            x192_add_u51(tot, p[0] + (p[1] << 16));
+            if (limbs) {
+                Exact192 a{0ULL, 0ULL, 0ULL, 0u};
+                if (lane >= 4 && lane < 10) {
+                    const int k = lane - 4;
+                    const unsigned long long lo = (k & 1) ? v << 32 : v, hi = (k & 1) ? v >> 32 : 0ULL;
+                    a.w0 = k < 2 ? lo : 0ULL;
+                    a.w1 = k < 2 ? hi : (k < 4 ? lo : 0ULL);
+                    a.w2 = k < 2 ? 0ULL : (k < 4 ? hi : lo);
+                }
+                a.nan = lane == 10 && v != 0ULL;
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) {
+                    const Exact192 b = x192_shfl_down(a, o);
+                    x192_add(a, b);
+                }
+                x192_add(tot, a);
             }
-            if (threadIdx.x == 0) {
+            if (lane == 0) {
                 const double t = x192_to_double(tot);
                 if (t > volfrac * (double)n) l1 = lmid;
                 else l2 = lmid;
                 s_l[0] = l1;
                 s_l[1] = l2;
                 s_l[2] = t;
+                s_l[3] = root(0.5 * (l2 + l1));
                 s_done = !((l2 - l1) / (l2 + l1) > 1e-3);
             }
         }
@@ -635,6 +704,8 @@ __global__ void __launch_bounds__(kOcThreads) k_oc_bisect(const float *x, const 
         l1 = s_l[0];
         l2 = s_l[1];
         sum = s_l[2];
+        rnext = s_l[3];
+        lnext = 0.5 * (l2 + l1);
         done = s_done != 0;
         nb++;
     }
@@ -651,7 +722,7 @@ __global__ void __launch_bounds__(kOcThreads) k_oc_bisect(const float *x, const 
     double mx = 0.0;
     for (int i = threadIdx.x; i < ne; i += blockDim.x) {
         const long long e = b0 + i;
-        const float v = oc_xnew(x[e], dc[e], pres, voidm, e, lmid, move);
+        const float v = __int_as_float(value(i));
         if (xold) mx = js_max(mx, fabs((double)v - (double)xold[e]));
         xnew[e] = v;
     }

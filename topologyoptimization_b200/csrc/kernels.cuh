@@ -5,14 +5,21 @@
 namespace tpo {
 
 // Bracket and result of one OC bisection; zeroed before the launch.
+struct OcWords {  // the sum of one bisection step over all blocks
+    unsigned long long piece[4];  // units of 2^-51, 2^-35, 2^-19, 2^-3
+    unsigned long long limb[6];   // units of 2^-149, 2^-117, ...: values the pieces do not hold
+    unsigned long long nan;
+};
+constexpr int kOcWords = sizeof(OcWords) / 8;
 struct OCState {
     double l1, l2, lmid, last_lmid, sum;
     unsigned long long change_bits;  // max |xnew - xold| as the bits of a non-negative double
     int done, nb;
     unsigned int bar;  // arrivals at the launch's grid barrier
     int err;           // the barrier's wait ran out
+    OcWords words[3];  // of the last steps and the next; zero at the start
 };
-constexpr int kOcThreads = 1024;
+constexpr int kOcThreads = 1024, kOcElemBytes = 16;
 
 // element stiffness
 __global__ void k_lk(double nu, double *Ke);
@@ -131,8 +138,7 @@ __global__ void __launch_bounds__(kOcThreads) k_oc_bisect(const float *x, const 
                                                           const uint8_t *__restrict__ pres,
                                                           const uint8_t *__restrict__ voidm, long long n, long long per,
                                                           int cap, double volfrac, double move, int max_bisections,
-                                                          OCState *s, unsigned long long *partials, const float *xold,
-                                                          float *xnew);
+                                                          OCState *s, const float *xold, float *xnew);
 
 __global__ void k_energy_wgsl(const float *__restrict__ U, const float *__restrict__ KE,
                               const int32_t *__restrict__ edofs, int nel, int es, float *__restrict__ out);
