@@ -633,6 +633,29 @@ def test_oc_bisect_edges(native, oracle, dims, kind):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("dims", [(15, 10, 10), (256, 148, 128), (257, 148, 128)])
+@pytest.mark.parametrize("scale", [1e-12, 1e-3, 1e9])
+def test_oc_bisect_steps_ahead(native, oracle, dims, scale):
+    """Multipliers that the bisection reaches after many, some and no halvings of its first
+    guess (steps taken four at a time between barriers, and the step that ends them at each
+    place among the four by the volume), with as many elements in each of 148 blocks as it is
+    done for (32,768), and more.  Bit for bit the oracle's, as the sum is exact."""
+    import torch
+    from topologyoptimization_b200 import Problem, mesh
+    n = int(np.prod(dims))
+    rng = np.random.default_rng(n)
+    x = rng.uniform(0.1, 0.5, n).astype(np.float32)
+    dc = (-scale * 10.0 ** rng.uniform(-2, 0, n)).astype(np.float32)
+    with Problem(*dims, mesh.fixed_mask(*dims, "left")) as P:
+        d_x, d_dc, d_xn = _dev(x), _dev(dc), torch.empty(n, dtype=torch.float32, device="cuda")
+        for vf in ((0.25, 0.27, 0.3, 0.33) if n == 1500 else (0.3,)):
+            xr, lmr, nbr = oracle.oc(x, vf, dc)
+            _, lm, nb = P.oc_update_dev(d_x, d_dc, d_xn, vf)
+            assert nb == nbr and lm == lmr
+            assert np.array_equal(d_xn.cpu().numpy(), xr)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("dims", [(4, 4, 4), (5, 5, 5), (7, 4, 11), (21, 13, 9), (60, 20, 20)])
 def test_galerkin_stencil_bitwise(native, oracle, dims):
     """Every dense level at the smallest grid with one, odd sizes on each axis and the largest

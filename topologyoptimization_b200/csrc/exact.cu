@@ -564,18 +564,20 @@ __device__ __forceinline__ int oc_bits(const OcElem &e, double rl) {
 // one and change = max |xnew - xold|.  Block b owns elements [b per, (b + 1) per); it keeps the
 // first `cap` of them in shared memory for all steps.  Each step every block sums its xnew
 // exactly and adds the sum to the step's words (integers: the total does not depend on the
-// order), and after the grid barrier every block reads the total and takes the same step.
+// order), and after a grid barrier every block reads the totals and takes the same steps.
 // Preserved and void elements contribute a constant, added once.
 //
 // A value in [2^-28, 2) is a multiple of 2^-51 and adds to one 64-bit sum, one in [2^-56, 2^-28) a
 // multiple of 2^-79 to another; what else there is goes through the 192-bit sum.
 //
-// One launch per step took 47-54 us a step whatever the size.  In this launch a step is bound by
+// One launch per step took 47-54 us a step whatever the size.  In this launch a pass is bound by
 // its barrier and two block reductions (3 to 4 us) up to 200,000 elements and by 25 instructions
-// an element beyond.  With a division and a root for every warp that holds an element between
-// its limits, and every block adding up all blocks' words, a call of nine steps took 74, 112,
-// 210, 347 us for 24,000, 524,288, 2.05M and 4.2M elements; it takes 67, 80, 118, 234 (the last
-// keeps only half of its elements in shared memory).
+// an element and step beyond.  With a division and a root for every warp that holds an element
+// between its limits, and every block adding up all blocks' words, a call of nine steps took
+// 74, 112, 210, 347 us for 24,000, 524,288, 2.05M and 4.2M elements; it takes 67, 80, 118, 234
+// (the last keeps only half of its elements in shared memory).  Several steps a pass take the
+// design update of 2.05M elements (some 40 steps, all kernels) from 0.82 to 0.75 ms; beyond
+// kOcAheadMax the steps that are dropped cost more than the barriers that are saved.
 __global__ void __launch_bounds__(kOcThreads) k_oc_bisect(const float *x, const float *dc,
                                                           const uint8_t *__restrict__ pres,
                                                           const uint8_t *__restrict__ voidm, long long n, long long per,
@@ -584,9 +586,9 @@ __global__ void __launch_bounds__(kOcThreads) k_oc_bisect(const float *x, const 
     extern __shared__ __align__(16) unsigned char smem_raw[];
     OcElem *sv = reinterpret_cast<OcElem *>(smem_raw);
     __shared__ Exact192 sh[32];
-    __shared__ unsigned piece[4][32];
+    __shared__ unsigned piece[kOcAhead][4][32];
     __shared__ double s_l[4];
-    __shared__ int s_done;
+    __shared__ int s_done, s_nb;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const long long b0 = blockIdx.x * per, b1 = min(n, b0 + per);
     const int ne = (int)max(0LL, b1 - b0);
@@ -606,109 +608,123 @@ __global__ void __launch_bounds__(kOcThreads) k_oc_bisect(const float *x, const 
     };
     // lmid^-1/2; NaN, which decides no element, for multipliers near the end of the range
     auto root = [](double l) { return l > 1e-290 ? rsqrt(l) : __longlong_as_double(0x7ff8000000000000LL); };
-    int nb = 0;
+    int nb = 0, pass = 0;
     bool done = !((l2 - l1) / (l2 + l1) > 1e-3);
-    double lnext = 0.5 * (l2 + l1), rnext = root(lnext);
     while (!done && nb < max_bisections) {
-        lmid = lnext;
-        rl = rnext;
-        Exact192 acc{0ULL, 0ULL, 0ULL, 0u};
-        unsigned long long fast = 0ULL, tiny = 0ULL;
-        bool rare = false;
-        int nf = 0;
-        for (int i = threadIdx.x; i < ne; i += blockDim.x) {
-            const int r = value(i);
-            const unsigned e = (unsigned)r >> 23;
-            const unsigned long long m = ((unsigned)r & 0x7fffffu) | 0x800000u;
-            if (e - 99u < 29u) {
-                fast += m << (e - 99u);
-            } else if (e - 71u < 28u) {
-                tiny += m << (e - 71u);
-            } else if (r != 0) {
-                x192_add_float(acc, __int_as_float(r));
-                rare = true;
+        // Steps between two barriers.  From 1e9 the multiplier falls by halves for some thirty steps
+        // until a sum exceeds the target: while it does, four at a time, each the one that
+        // follows if the sum before it is small; the step that is not drops those after it.
+        const int nk = l1 == 0.0 && nb > 0 && per <= kOcAheadMax ? min(kOcAhead, max_bisections - nb) : 1;
+        OcWords *words = s->words[pass % 3];
+        for (int k = 0; k < nk; k++) {
+            lmid = 0.5 * ((k == 0 ? l2 : lmid) + l1);
+            rl = root(lmid);
+            Exact192 acc{0ULL, 0ULL, 0ULL, 0u};
+            unsigned long long fast = 0ULL, tiny = 0ULL;
+            bool rare = false;
+            int nf = 0;
+            for (int i = threadIdx.x; i < ne; i += blockDim.x) {
+                const int r = value(i);
+                const unsigned e = (unsigned)r >> 23;
+                const unsigned long long m = ((unsigned)r & 0x7fffffu) | 0x800000u;
+                if (e - 99u < 29u) {
+                    fast += m << (e - 99u);
+                } else if (e - 71u < 28u) {
+                    tiny += m << (e - 71u);
+                } else if (r != 0) {
+                    x192_add_float(acc, __int_as_float(r));
+                    rare = true;
+                }
+                if (++nf == kFastFlush) {
+                    x192_add_u51(acc, fast);
+                    x192_add_u79(acc, tiny);
+                    fast = tiny = 0ULL;
+                    rare = true;
+                    nf = 0;
+                }
             }
-            if (++nf == kFastFlush) {
-                x192_add_u51(acc, fast);
+            OcWords *w = words + k;
+#pragma unroll
+            for (int q = 0; q < 4; q++) {  // 16 bits of every thread's sum at a time
+                const unsigned p = __reduce_add_sync(0xffffffffu, (unsigned)(fast >> (16 * q)) & 0xffffu);
+                if (lane == 0) piece[k][q][wid] = p;
+            }
+            if (__syncthreads_or(rare || tiny != 0ULL)) {
                 x192_add_u79(acc, tiny);
-                fast = tiny = 0ULL;
-                rare = true;
-                nf = 0;
-            }
-        }
-        OcWords *w = &s->words[nb % 3];
-#pragma unroll
-        for (int k = 0; k < 4; k++) {  // 16 bits of every thread's sum at a time
-            const unsigned p = __reduce_add_sync(0xffffffffu, (unsigned)(fast >> (16 * k)) & 0xffffu);
-            if (lane == 0) piece[k][wid] = p;
-        }
-        if (__syncthreads_or(rare || tiny != 0ULL)) {
-            x192_add_u79(acc, tiny);
-            acc = x192_block_sum(acc, sh);
-            if (threadIdx.x == 0) {
-                const unsigned long long l[3] = {acc.w0, acc.w1, acc.w2};
-                for (int k = 0; k < 3; k++) {
-                    if (!l[k]) continue;
-                    atomicAdd(&w->limb[2 * k], l[k] & 0xffffffffULL);
-                    atomicAdd(&w->limb[2 * k + 1], l[k] >> 32);
+                acc = x192_block_sum(acc, sh);
+                if (threadIdx.x == 0) {
+                    const unsigned long long l[3] = {acc.w0, acc.w1, acc.w2};
+                    for (int q = 0; q < 3; q++) {
+                        if (!l[q]) continue;
+                        atomicAdd(&w->limb[2 * q], l[q] & 0xffffffffULL);
+                        atomicAdd(&w->limb[2 * q + 1], l[q] >> 32);
+                    }
+                    if (acc.nan) atomicAdd(&w->nan, 1ULL);
                 }
-                if (acc.nan) atomicAdd(&w->nan, 1ULL);
+            }
+            if (wid < 4) {
+                const unsigned p =
+                    __reduce_add_sync(0xffffffffu, lane < (int)(blockDim.x >> 5) ? piece[k][wid][lane] : 0u);
+                if (lane == 0 && p) atomicAdd(&w->piece[wid], (unsigned long long)p);
             }
         }
-        if (wid < 4) {
-            const unsigned p = __reduce_add_sync(0xffffffffu, lane < (int)(blockDim.x >> 5) ? piece[wid][lane] : 0u);
-            if (lane == 0 && p) atomicAdd(&w->piece[wid], (unsigned long long)p);
-        }
-        if (!grid_barrier(&s->bar, (unsigned)(nb + 1) * gridDim.x, &s->err)) return;
-        // the words of the step before are read everywhere: clear them for the step after the next
-        if (blockIdx.x == 0 && wid == 1 && lane < kOcWords)
-            reinterpret_cast<unsigned long long *>(&s->words[(nb + 2) % 3])[lane] = 0ULL;
+        if (!grid_barrier(&s->bar, (unsigned)(pass + 1) * gridDim.x, &s->err)) return;
+        // the words of the pass before are read everywhere: clear them for the pass after the next
+        if (blockIdx.x == 0 && wid == 1)
+            for (int i = lane; i < kOcAhead * kOcWords; i += 32)
+                reinterpret_cast<unsigned long long *>(s->words[(pass + 2) % 3])[i] = 0ULL;
         if (wid == 0) {
-            const unsigned long long v =
-                lane < kOcWords ? __ldcg(reinterpret_cast<unsigned long long *>(w) + lane) : 0ULL;
-            const bool limbs = __any_sync(0xffffffffu, lane >= 4 && v != 0ULL);
-            unsigned long long p[4];
+            double t = 0.0;
+            if (lane < nk) {  // lane k adds up step k
+                unsigned long long v[kOcWords];
 #pragma unroll
-            for (int k = 0; k < 4; k++) p[k] = __shfl_sync(0xffffffffu, v, k);
-            Exact192 tot{0ULL, 0ULL, (p[2] + (p[3] << 16)) << 2, 0u};  // 2^-19 = 2^130 2^-149
-            x192_add_u51(tot, p[0] + (p[1] << 16));
-            if (limbs) {
-                Exact192 a{0ULL, 0ULL, 0ULL, 0u};
-                if (lane >= 4 && lane < 10) {
-                    const int k = lane - 4;
-                    const unsigned long long lo = (k & 1) ? v << 32 : v, hi = (k & 1) ? v >> 32 : 0ULL;
-                    a.w0 = k < 2 ? lo : 0ULL;
-                    a.w1 = k < 2 ? hi : (k < 4 ? lo : 0ULL);
-                    a.w2 = k < 2 ? 0ULL : (k < 4 ? hi : lo);
-                }
-                a.nan = lane == 10 && v != 0ULL;
+                for (int i = 0; i < kOcWords; i++)
+                    v[i] = __ldcg(reinterpret_cast<unsigned long long *>(words + lane) + i);
+                // 2^-19 = 2^130 2^-149
+                Exact192 tot{0ULL, 0ULL, (v[2] + (v[3] << 16)) << 2, (unsigned)(v[10] != 0ULL)};
+                x192_add_u51(tot, v[0] + (v[1] << 16));
 #pragma unroll
-                for (int o = 16; o > 0; o >>= 1) {
-                    const Exact192 b = x192_shfl_down(a, o);
-                    x192_add(a, b);
+                for (int q = 0; q < 6; q++) {
+                    const unsigned long long lo = (q & 1) ? v[4 + q] << 32 : v[4 + q], hi = (q & 1) ? v[4 + q] >> 32 : 0ULL;
+                    const Exact192 a{q < 2 ? lo : 0ULL, q < 2 ? hi : (q < 4 ? lo : 0ULL), q < 2 ? 0ULL : (q < 4 ? hi : lo), 0u};
+                    if (v[4 + q]) x192_add(tot, a);
                 }
-                x192_add(tot, a);
+                t = x192_to_double(tot);
             }
+            double tk[kOcAhead];
+#pragma unroll
+            for (int k = 0; k < kOcAhead; k++) tk[k] = __shfl_sync(0xffffffffu, t, k);
             if (lane == 0) {
-                const double t = x192_to_double(tot);
-                if (t > volfrac * (double)n) l1 = lmid;
-                else l2 = lmid;
+#pragma unroll
+                for (int k = 0; k < kOcAhead; k++) {
+                    if (k >= nk || done) break;
+                    lmid = 0.5 * (l2 + l1);
+                    sum = tk[k];
+                    const bool up = sum > volfrac * (double)n;
+                    if (up) l1 = lmid;
+                    else l2 = lmid;
+                    nb++;
+                    done = !((l2 - l1) / (l2 + l1) > 1e-3);
+                    if (up) break;
+                }
                 s_l[0] = l1;
                 s_l[1] = l2;
-                s_l[2] = t;
-                s_l[3] = root(0.5 * (l2 + l1));
-                s_done = !((l2 - l1) / (l2 + l1) > 1e-3);
+                s_l[2] = sum;
+                s_l[3] = lmid;
+                s_nb = nb;
+                s_done = done;
             }
         }
         __syncthreads();
         l1 = s_l[0];
         l2 = s_l[1];
         sum = s_l[2];
-        rnext = s_l[3];
-        lnext = 0.5 * (l2 + l1);
+        lmid = s_l[3];
+        nb = s_nb;
         done = s_done != 0;
-        nb++;
+        pass++;
     }
+    rl = root(lmid);
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         s->l1 = l1;
         s->l2 = l2;

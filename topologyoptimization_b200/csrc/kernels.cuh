@@ -11,13 +11,15 @@ struct OcWords {  // the sum of one bisection step over all blocks
     unsigned long long nan;
 };
 constexpr int kOcWords = sizeof(OcWords) / 8;
+constexpr int kOcAhead = 4;            // bisection steps between two grid barriers at most
+constexpr long long kOcAheadMax = 32768;  // elements a block up to which steps are taken ahead
 struct OCState {
     double l1, l2, lmid, last_lmid, sum;
     unsigned long long change_bits;  // max |xnew - xold| as the bits of a non-negative double
     int done, nb;
     unsigned int bar;  // arrivals at the launch's grid barrier
     int err;           // the barrier's wait ran out
-    OcWords words[3];  // of the last steps and the next; zero at the start
+    OcWords words[3][kOcAhead];  // of the last passes and the next; zero at the start
 };
 constexpr int kOcThreads = 1024, kOcElemBytes = 16;
 
