@@ -149,3 +149,29 @@ def test_2d_one_launch_solve(native, oracle, dims):
     assert np.abs(r["complianceHistory"][:n] / ro["compliance"][:n] - 1).max() < 1e-7
     if ro["iterations"] == r["iterations"]:
         assert np.abs(r["densities2D"] - ro["x"]).max() < 1e-5
+
+
+@pytest.mark.gpu
+def test_2d_more_void_than_the_target_leaves(native, oracle):
+    """Void elements on most (77%) of the domain and a volume fraction of 0.3: the target cannot be
+    exceeded, and two SIMP iterations still keep preserved elements at 1 and void ones at 0.
+    The suite's bound on x of short 2D runs."""
+    from topologyoptimization_b200 import mesh
+    from topologyoptimization_b200.worker2d import TopologyOptimizerWorker
+    nx, ny = 30, 10
+    pres = np.zeros(nx * ny, np.uint8)
+    pres[mesh.constraint_elements2d(nx, ny, "left")] = 1
+    pres[mesh.force_elements2d(nx, ny, "down")] = 1
+    # the two rows that carry the load stay free
+    void = np.zeros((nx, ny), np.uint8)
+    void[:, :ny - 2] = 1
+    void = void.reshape(-1) * (1 - pres)
+    ro = oracle.simp2d(nx, ny, mesh.load_vector2d(nx, ny, "down"), mesh.fixed_mask2d(nx, ny, "left"), pres, void, max_iter=2,
+                       use_projection=1)
+    r = TopologyOptimizerWorker().optimize({"nx": nx, "ny": ny},
+                                           dict(volumeFraction=0.3, maxIterations=2, penaltyFactor=3.0, filterRadius=1.5,
+                                                preservedElements=pres, voidElements=void))
+    assert r["iterations"] == ro["iterations"]
+    assert np.isfinite(ro["x"]).all()
+    assert np.abs(r["densities2D"] - ro["x"]).max() < 1e-5
+    assert (r["densities2D"].reshape(-1)[pres == 1] == 1).all()

@@ -768,3 +768,31 @@ def test_small_grid_apply(native, oracle, dims):
             P.set_load(F[k])
             P.solve_dev(V, o)
             assert rel_inf(U[k].cpu().numpy(), V.cpu().numpy()) < 1e-10
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dims,volfrac,share_void,x0", [((10, 10, 1), 0.5, 0.05, 0.1), ((15, 10, 10), 0.3, 0.8, None),
+                                                        ((60, 20, 20), 1.0, 0.1, None), ((160, 128, 104), 0.5, 0.6, None)])
+def test_oc_unreachable_volume_keeps_masks(native, oracle, dims, volfrac, share_void, x0):
+    """A volume target that no multiplier exceeds: the bracket halves to zero, where lambda^-1/2 is
+    no number any more, and preserved and void elements stay 1 and 0 all the same (void ones
+    with x = 0 too, whose product with it is NaN).  The last size keeps some of its elements
+    outside shared memory.  Bit for bit the oracle's."""
+    import torch
+    from topologyoptimization_b200 import Problem, mesh
+    n = int(np.prod(dims))
+    rng = np.random.default_rng(n)
+    x = np.full(n, x0, np.float32) if x0 else rng.uniform(0.05, 1.0, n).astype(np.float32)
+    dc = (-(10.0 ** rng.uniform(-3, 3, n))).astype(np.float32)
+    pres = (rng.random(n) < 0.05).astype(np.uint8)
+    void = (rng.random(n) < share_void).astype(np.uint8) * (1 - pres)
+    x[(void == 1) & (rng.random(n) < 0.5)] = 0.0
+    with np.errstate(all="ignore"):
+        xr, lmr, nbr = oracle.oc(x, volfrac, dc, preserved=pres, void=void)
+    assert nbr > 1000 and (xr[pres == 1] == 1).all() and (xr[void == 1] == 0).all()
+    with Problem(*dims, mesh.fixed_mask(*dims, "left")) as P:
+        d_xn = torch.empty(n, dtype=torch.float32, device="cuda")
+        _, lm, nb = P.oc_update_dev(_dev(x), _dev(dc), d_xn, volfrac, d_preserved=_dev(pres), d_void=_dev(void))
+        xn = d_xn.cpu().numpy()
+    assert nb == nbr and lm == lmr
+    assert np.array_equal(xn, xr, equal_nan=True)

@@ -603,10 +603,12 @@ __global__ void __launch_bounds__(kOcThreads) k_oc_bisect(const float *x, const 
     double l1 = 0.0, l2 = 1e9, lmid = 0.0, rl = 0.0, sum = 0.0;
     auto value = [&](int i) {  // bits of xnew(lmid)
         int r = oc_bits(i < ns ? sv[i] : elem(i), rl);
-        if (r < 0) r = __float_as_int(oc_xnew(x[b0 + i], dc[b0 + i], nullptr, nullptr, 0, lmid, move));
+        // with the masks: without a root (lmid near 0) no element is decided, masked ones neither
+        if (r < 0) r = __float_as_int(oc_xnew(x[b0 + i], dc[b0 + i], pres, voidm, b0 + i, lmid, move));
         return r;
     };
-    // lmid^-1/2; NaN, which decides no element, for multipliers near the end of the range
+    // lmid^-1/2; NaN, which decides no element, for multipliers near the end of the range (where a
+    // bracket ends whose volume target no multiplier exceeds)
     auto root = [](double l) { return l > 1e-290 ? rsqrt(l) : __longlong_as_double(0x7ff8000000000000LL); };
     int nb = 0, pass = 0;
     bool done = !((l2 - l1) / (l2 + l1) > 1e-3);
