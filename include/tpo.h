@@ -273,6 +273,11 @@ void *tpo_stream(tpo_problem *p);
  * The library's own stream is ordered with the legacy default stream; a caller's
  * non-blocking stream is not, so the caller orders its own work on it. */
 tpo_status tpo_set_stream(tpo_problem *p, void *stream);
+/* Limits of the kernels that run a whole loop on the device (Jacobi-PCG of small grids, OC
+ * bisection): PCG iterations of one launch (even, default 4096; the host launches again
+ * until the solve is done), and polls of a wait inside a launch (default 2^22, some
+ * seconds) after which the call returns TPO_TIMEOUT.  The problem stays usable. */
+tpo_status tpo_set_launch_limits(tpo_problem *p, int32_t iterations, uint32_t polls);
 
 /* ---- batched solves (the chosen form's block MG-PCG; the reference solves load cases one
  * at a time) ------------------------------------------------------------------------- */

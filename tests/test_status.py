@@ -104,3 +104,62 @@ def test_bisection_cap_is_timeout(native):
         assert e.value.status == N.TPO_TIMEOUT
         ch, lm, nb = P.oc_update_dev(x, dc, xn, 0.3)
         assert nb > 5 and ch > 0
+
+
+def _jacobi(P, F, n=60):
+    from topologyoptimization_b200 import _native as N
+    P.set_load(F)
+    return P.solve(None, precond=N.PREC_JACOBI, max_iter=n, tol=0.0, warm_start=0, ref_epsilon=0)
+
+
+def test_barrier_wait_is_timeout_and_leaves_the_handle_usable(native):
+    """Barrier waits of a single poll run out (some 140 blocks do not all arrive within one):
+    TPO_TIMEOUT from the Jacobi solve and from the OC update, and with the limit back both
+    give what a handle gives that never saw one."""
+    import torch
+    from topologyoptimization_b200 import Problem, mesh
+    from topologyoptimization_b200 import _native as N
+    dims = (60, 20, 20)
+    fixed = mesh.fixed_mask(*dims, "left")
+    rng = np.random.default_rng(4)
+    x = rng.uniform(0.2, 1, 24000).astype(np.float32)
+    F = rng.standard_normal(len(fixed)) * (fixed == 0)
+    d_x = torch.from_numpy(x).cuda()
+    d_dc = torch.from_numpy((-rng.uniform(0.5, 2, 24000)).astype(np.float32)).cuda()
+    d_xn, d_ref = torch.empty_like(d_x), torch.empty_like(d_x)
+    with Problem(*dims, fixed) as P, Problem(*dims, fixed) as Q:
+        for A in (P, Q):
+            A.set_densities(x, 3.0)
+        P.set_launch_limits(polls=1)
+        for call in (lambda: _jacobi(P, F), lambda: P.oc_update_dev(d_x, d_dc, d_xn, 0.3)):
+            with pytest.raises(N.TpoError) as e:
+                call()
+            assert e.value.status == N.TPO_TIMEOUT
+        P.set_launch_limits()
+        U, info = _jacobi(P, F)
+        Ur, infor = _jacobi(Q, F)
+        assert info.iterations == infor.iterations == 60 and np.array_equal(U, Ur)
+        assert P.oc_update_dev(d_x, d_dc, d_xn, 0.3) == Q.oc_update_dev(d_x, d_dc, d_ref, 0.3)
+        assert torch.equal(d_xn, d_ref)
+
+
+@pytest.mark.parametrize("dims", [(4, 4, 4), (40, 22, 20)])
+def test_jacobi_solve_split_over_launches(native, dims):
+    """The one-launch Jacobi solve handed over between launches of 2, 8 and 64 iterations: bit for
+    bit the solve in one (19,803 nodes: five a lane), at a count that is no multiple of them."""
+    from topologyoptimization_b200 import Problem, mesh
+    from topologyoptimization_b200 import _native as N
+    fixed = mesh.fixed_mask(*dims, "left")
+    rng = np.random.default_rng(6)
+    F = rng.standard_normal(len(fixed)) * (fixed == 0)
+    with Problem(*dims, fixed) as P:
+        P.set_densities(rng.uniform(0.2, 1, int(np.prod(dims))).astype(np.float32), 3.0)
+        U, info = _jacobi(P, F, 77)
+        for iterations in (2, 8, 64):
+            P.set_launch_limits(iterations=iterations)
+            V, infov = _jacobi(P, F, 77)
+            assert infov.iterations == info.iterations and np.array_equal(U, V)
+        for bad in (dict(iterations=3), dict(iterations=0), dict(polls=0)):
+            with pytest.raises(N.TpoError) as e:
+                P.set_launch_limits(**bad)
+            assert e.value.status == N.TPO_BAD_ARG

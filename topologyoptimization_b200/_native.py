@@ -125,6 +125,7 @@ _SIGS = {
     "tpo_volumetric_snapshot": (C.c_int, [_P, _P, _P]),
     "tpo_stream": (C.c_void_p, [_P]),
     "tpo_set_stream": (C.c_int, [_P, _P]),
+    "tpo_set_launch_limits": (C.c_int, [_P, C.c_int32, C.c_uint32]),
     "tpo_solve_multi_dev": (C.c_int, [_P, _P, C.c_int32, _P, _P, _P]),
     "tpo_set_spring": (C.c_int, [_P, C.c_int64, C.c_double]),
     "tpo_forward_dev": (C.c_int, [_P, _P, _P, _P, _P, _P, _P]),

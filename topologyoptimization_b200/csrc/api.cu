@@ -679,6 +679,9 @@ struct tpo_problem {
     float *stress = nullptr;
     unsigned long long *stress_max = nullptr;
     int stress_valid = 0;
+    // limits of the cooperative launches (tpo_set_launch_limits)
+    int coop_iters = kCoopIters;
+    unsigned wait_polls = kBarrierPolls;
     // captured PCG iteration chunks
     cudaGraphExec_t gexec[kIterModes] = {};
     int gchunk[kIterModes] = {};
@@ -1409,19 +1412,19 @@ void run_iterations(tpo_problem *P, int mode, CGState *st, CGState *st_host, int
     }
 }
 
-// Cooperative launches of kCoopIters iterations each until the state says done (`launch` makes
-// one); the host reads the state between them.
+// Cooperative launches of `iters` iterations each until the state says done (`launch` makes
+// one); the host reads the state between them.  A wait that ran out ends this solve alone.
 template <class F>
-void run_coop(cudaStream_t s, CGState *st, CGState *st_host, int max_iter, F &&launch) {
-    const long long max_launch = std::max(0, max_iter) / kCoopIters + 2;
+void run_coop(cudaStream_t s, CGState *st, CGState *st_host, int max_iter, int iters, F &&launch) {
+    const long long max_launch = std::max(0, max_iter) / iters + 2;
     for (long long c = 0;; c++) {
         if (c > max_launch) fail(TPO_CUDA_ERROR, "PCG state machine did not terminate");
-        CK(cudaMemsetAsync(&st->bar, 0, sizeof(unsigned), s));
+        CK(cudaMemsetAsync(&st->wait, 0, sizeof(CoopWait), s));
         launch();
         CKL();
         CK(cudaMemcpyAsync(st_host, st, sizeof(CGState), cudaMemcpyDeviceToHost, s));
         CK(cudaStreamSynchronize(s));
-        if (st_host->bar_err) fail(TPO_TIMEOUT, "a grid barrier of the Jacobi-PCG ran out");
+        if (st_host->wait.err) fail(TPO_TIMEOUT, "a grid barrier of the Jacobi-PCG ran out");
         if (st_host->done) return;
     }
 }
@@ -1452,8 +1455,9 @@ bool jacobi_coop(tpo_problem *P, int max_iter) {
     KeParam<double> ke = P->ke;
     Grid gg = g;
     Level &L0 = P->L[0];
-    void *args[] = {&ke, &gg, &L0.Eact, &L0.invD, &L0.fixed, &P->U, &P->r, &P->z, &P->p, &P->Ap, &P->st, &P->partials};
-    run_coop(P->s, P->st, P->st_host, max_iter, [&] {
+    void *args[] = {&ke, &gg, &L0.Eact, &L0.invD, &L0.fixed, &P->U, &P->r, &P->z, &P->p, &P->Ap, &P->st, &P->partials,
+                    &P->coop_iters, &P->wait_polls};
+    run_coop(P->s, P->st, P->st_host, max_iter, P->coop_iters, [&] {
         CK(cudaLaunchCooperativeKernel(k, dim3(blocks), dim3(kCoop3Threads), args, smem, P->s));
     });
     return true;
@@ -1721,6 +1725,7 @@ struct OcCtx {
     cudaStream_t s;
     OCState *oc, *oc_host;
     long long n;
+    unsigned polls;
 };
 
 // One cooperative launch: a block of kOcThreads per SM at most, each keeping as many of its
@@ -1742,7 +1747,8 @@ void run_oc_ctx(const OcCtx &c, const float *d_x, double volfrac, const float *d
     CK(cudaMemsetAsync(c.oc, 0, sizeof(OCState), c.s));
     long long n = c.n;
     OCState *oc = c.oc;
-    void *args[] = {&d_x, &d_dc, &pres, &voidm, &n, &per, &cap, &volfrac, &move, &max_bisections, &oc, &d_xold, &d_xnew};
+    unsigned polls = c.polls;
+    void *args[] = {&d_x, &d_dc, &pres, &voidm, &n, &per, &cap, &volfrac, &move, &max_bisections, &oc, &d_xold, &d_xnew, &polls};
     CK(cudaLaunchCooperativeKernel((const void *)k_oc_bisect, dim3((unsigned)blocks), dim3(kOcThreads), args, smem, c.s));
     CKL();
     CK(cudaMemcpyAsync(c.oc_host, c.oc, sizeof(OCState), cudaMemcpyDeviceToHost, c.s));
@@ -1760,7 +1766,7 @@ void run_oc_ctx(const OcCtx &c, const float *d_x, double volfrac, const float *d
 void run_oc(tpo_problem *P, const float *d_x, double volfrac, const float *d_dc, const uint8_t *pres,
             const uint8_t *voidm, float *d_xnew, const float *d_xold, double *lmid, int *nb, double *change,
             double move = 0.2, int max_bisections = 1280) {
-    const OcCtx c{P->s, P->oc, P->oc_host, P->g.nel};
+    const OcCtx c{P->s, P->oc, P->oc_host, P->g.nel, P->wait_polls};
     run_oc_ctx(c, d_x, volfrac, d_dc, pres, voidm, d_xnew, d_xold, lmid, nb, change, move, max_bisections);
 }
 
@@ -1907,6 +1913,16 @@ tpo_status tpo_set_stream(tpo_problem *p, void *stream) {
         if (!p) fail(TPO_BAD_ARG, "problem is null");
         CK(cudaStreamSynchronize(p->s));
         p->s = stream ? (cudaStream_t)stream : p->own;
+    });
+}
+
+tpo_status tpo_set_launch_limits(tpo_problem *p, int32_t iterations, uint32_t polls) {
+    return guard([&] {
+        if (!p) fail(TPO_BAD_ARG, "problem is null");
+        if (iterations < 2 || iterations % 2) fail(TPO_BAD_ARG, "iterations of a launch must be even and positive");
+        if (polls < 1) fail(TPO_BAD_ARG, "polls must be positive");
+        p->coop_iters = iterations;
+        p->wait_polls = polls;
     });
 }
 
@@ -2945,8 +2961,11 @@ tpo_status tpo_simp2d_step_dev(tpo_problem2d *p, const tpo_simp2d_opts *o, float
             // and the dot products keep the order of the separate kernels.
             int nx = p->nelx, ny = p->nely;
             double th = thresh;
-            void *args[] = {&p->dKe, &nx, &ny, &p->E, &th, &p->invD, &p->fixed, &p->U, &p->r, &p->z, &p->p, &p->Ap, &p->st, &p->partials};
-            run_coop(s, p->st, p->st_host, cgMax, [&] {
+            int iters = kCoopIters;
+            unsigned polls = kBarrierPolls;
+            void *args[] = {&p->dKe, &nx, &ny, &p->E, &th, &p->invD, &p->fixed, &p->U, &p->r, &p->z, &p->p, &p->Ap, &p->st,
+                            &p->partials, &iters, &polls};
+            run_coop(s, p->st, p->st_host, cgMax, iters, [&] {
                 CK(cudaLaunchCooperativeKernel((const void *)k_cg_coop2, dim3(cb), dim3(kCoop2Threads), args, 0, s));
             });
             h = *p->st_host;
@@ -3012,7 +3031,7 @@ tpo_status tpo_simp2d_step_dev(tpo_problem2d *p, const tpo_simp2d_opts *o, float
         CK(cudaStreamSynchronize(s));
         const double compliance = p->scal_host[0];
         double change = 0.0;
-        const OcCtx c{s, p->oc, p->oc_host, ne};
+        const OcCtx c{s, p->oc, p->oc_host, ne, kBarrierPolls};
         run_oc_ctx(c, p->xold, o->volfrac, p->dcn, d_preserved, d_void, d_x, p->xold, nullptr, nullptr, &change, 0.2,
                    1280);
         if (info) {

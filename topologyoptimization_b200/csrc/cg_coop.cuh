@@ -18,7 +18,10 @@
 
 namespace tpo {
 
-constexpr int kCoopIters = 4096;  // iterations of one launch; the host launches again if need be
+// Iterations of one launch unless the caller sets another even number; the host launches again if
+// need be.  Even: p is back in its first array when a launch ends without being done.
+constexpr int kCoopIters = 4096;
+static_assert(kCoopIters % 2 == 0, "p alternates between two arrays");
 
 // Scalars of the recurrence, the same in every block.
 struct CoopScalars {
@@ -102,7 +105,7 @@ __global__ void __launch_bounds__(kCoop3Threads) k_cg_coop3(const __grid_constan
                                                             const double *__restrict__ invD,
                                                             const uint8_t *__restrict__ fixed, double *U, double *r,
                                                             double *z, double *pa, double *pb, CGState *st,
-                                                            double *parts) {
+                                                            double *parts, int iters, unsigned polls) {
     constexpr int NT = 32 * M, SEG = (NT + 2) * 3, Q = (3 * NT + kCoop3Threads - 1) / kCoop3Threads;
     constexpr int kLoads = (9 * SEG + kCoop3Threads - 1) / kCoop3Threads, kBatch = 6;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -145,7 +148,7 @@ __global__ void __launch_bounds__(kCoop3Threads) k_cg_coop3(const __grid_constan
     double *pold = pa, *pnew = pb;
     unsigned epoch = 0;
     bool ok = true;
-    while (!s.done && s.it - it0 < kCoopIters) {
+    while (!s.done && s.it - it0 < iters) {
         // 1: p at the block's nodes and their neighbours, the loads of several in flight together
 #pragma unroll
         for (int l0 = 0; l0 < kLoads; l0 += kBatch) {
@@ -203,7 +206,7 @@ __global__ void __launch_bounds__(kCoop3Threads) k_cg_coop3(const __grid_constan
         }
         block_sum<1>(v1, sh);
         if (tid == 0) parts[blockIdx.x] = v1[0];
-        if (!(ok = grid_barrier(&st->bar, ++epoch * nb, &st->bar_err))) break;
+        if (!(ok = grid_barrier(&st->wait.bar, ++epoch * nb, &st->wait.err, polls))) break;
         double t1[1];
         coop_total<1>(parts, nb, sh2, t1);
         if (!coop_alpha(s, t1[0], eps, st, blockIdx.x == 0 && tid == 0)) break;
@@ -224,7 +227,7 @@ __global__ void __launch_bounds__(kCoop3Threads) k_cg_coop3(const __grid_constan
             parts[nb + blockIdx.x] = v2[0];
             parts[2 * nb + blockIdx.x] = v2[1];
         }
-        if (!(ok = grid_barrier(&st->bar, ++epoch * nb, &st->bar_err))) break;
+        if (!(ok = grid_barrier(&st->wait.bar, ++epoch * nb, &st->wait.err, polls))) break;
         double t2[2];
         coop_total<2>(parts + nb, nb, sh2, t2);
         coop_beta(s, t2[0], t2[1], eps, tolSq, maxIter, st, blockIdx.x == 0 && tid == 0);

@@ -74,6 +74,12 @@ inline Grid make_grid(int nelx, int nely, int nelz) {
     return g;
 }
 
+// Barrier state of a cooperative launch.
+struct CoopWait {
+    unsigned int bar;  // arrivals
+    int err;           // a wait ran out
+};
+
 // Scalars of one PCG solve, resident in device memory so that no iteration needs a
 // host round trip.  Kernels of an iteration return at once when done != 0.
 struct CGState {
@@ -91,8 +97,7 @@ struct CGState {
     double rr32, maxr2, delta2;
     int do_update, n_updates;
     unsigned int counters[8];
-    unsigned int bar;  // arrivals at the grid barriers of a cooperative launch (zeroed before it)
-    int bar_err;       // one of its waits ran out
+    CoopWait wait;  // of a cooperative launch, zeroed before each
 };
 
 // Convergence decision after an iteration that produced ||r||^2 in st->rr, with the
@@ -245,11 +250,12 @@ __device__ __forceinline__ bool grid_sum(double (&v)[NV], double *partials, unsi
 
 // ---- grid barrier of a cooperative launch ---------------------------------------
 // Every block arrives once per epoch; `target` is epoch * blocks.  All blocks are resident (a
-// cooperative launch), so the wait ends; a wait of some seconds sets *err instead, and the
-// kernel returns.  What a block wrote before the barrier is visible to every block after it
-// (reads of such data use __ldcg or volatile accesses: L1 is not coherent).
-constexpr unsigned kBarrierSpins = 1u << 22;
-__device__ __forceinline__ bool grid_barrier(unsigned *count, unsigned target, int *err) {
+// cooperative launch), so the wait ends; one of more than `polls` polls (some seconds' worth
+// unless the caller sets less) sets *err instead, and the kernel returns.  What a block wrote
+// before the barrier is visible to every block after it (reads of such data use __ldcg or
+// volatile accesses: L1 is not coherent).
+constexpr unsigned kBarrierPolls = 1u << 22;
+__device__ __forceinline__ bool grid_barrier(unsigned *count, unsigned target, int *err, unsigned polls) {
     __shared__ int s_ok;
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -258,7 +264,7 @@ __device__ __forceinline__ bool grid_barrier(unsigned *count, unsigned target, i
         unsigned v, spins = 0;
         do {
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(count) : "memory");
-        } while ((int)(v - target) < 0 && ++spins < kBarrierSpins);
+        } while ((int)(v - target) < 0 && ++spins < polls);
         s_ok = (int)(v - target) >= 0;
         if (!s_ok) atomicExch(err, 1);
     }

@@ -582,7 +582,7 @@ __global__ void __launch_bounds__(kOcThreads) k_oc_bisect(const float *x, const 
                                                           const uint8_t *__restrict__ pres,
                                                           const uint8_t *__restrict__ voidm, long long n, long long per,
                                                           int cap, double volfrac, double move, int max_bisections,
-                                                          OCState *s, const float *xold, float *xnew) {
+                                                          OCState *s, const float *xold, float *xnew, unsigned polls) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     OcElem *sv = reinterpret_cast<OcElem *>(smem_raw);
     __shared__ Exact192 sh[32];
@@ -670,7 +670,7 @@ __global__ void __launch_bounds__(kOcThreads) k_oc_bisect(const float *x, const 
                 if (lane == 0 && p) atomicAdd(&w->piece[wid], (unsigned long long)p);
             }
         }
-        if (!grid_barrier(&s->bar, (unsigned)(pass + 1) * gridDim.x, &s->err)) return;
+        if (!grid_barrier(&s->bar, (unsigned)(pass + 1) * gridDim.x, &s->err, polls)) return;
         // the words of the pass before are read everywhere: clear them for the pass after the next
         if (blockIdx.x == 0 && wid == 1)
             for (int i = lane; i < kOcAhead * kOcWords; i += 32)
@@ -925,7 +925,7 @@ __global__ void __launch_bounds__(kCoop2Threads) k_cg_coop2(const double *__rest
                                                             const double *__restrict__ invD,
                                                             const uint8_t *__restrict__ fixed, double *U, double *r,
                                                             double *z, double *pa, double *pb, CGState *st,
-                                                            double *parts) {
+                                                            double *parts, int iters, unsigned polls) {
     constexpr int NT = kCoop2Threads / 2, SEG = (NT + 2) * 2;
     __shared__ double sp[3 * SEG], sK[64], sh[64], sh2[16];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -973,7 +973,7 @@ __global__ void __launch_bounds__(kCoop2Threads) k_cg_coop2(const double *__rest
             }
         }
     };
-    while (!s.done && s.it - it0 < kCoopIters) {
+    while (!s.done && s.it - it0 < iters) {
         constexpr int kLoads = (3 * SEG + kCoop2Threads - 1) / kCoop2Threads;
         double zv[kLoads], pv[kLoads];
 #pragma unroll
@@ -1017,7 +1017,7 @@ __global__ void __launch_bounds__(kCoop2Threads) k_cg_coop2(const double *__rest
         if (fx) ap = 0.0;
         if (own) pnew[d] = pd;
         part_sums(own ? pd * ap : 0.0, 0.0, 1, parts);
-        if (!(ok = grid_barrier(&st->bar, ++epoch * gridDim.x, &st->bar_err))) break;
+        if (!(ok = grid_barrier(&st->wait.bar, ++epoch * gridDim.x, &st->wait.err, polls))) break;
         double t1[1];
         coop_total<1>(parts, nparts, sh2, t1);
         if (!coop_alpha(s, t1[0], eps, st, blockIdx.x == 0 && tid == 0)) break;
@@ -1026,7 +1026,7 @@ __global__ void __launch_bounds__(kCoop2Threads) k_cg_coop2(const double *__rest
         Ud = fma(s.alpha, pd, Ud);
         if (own) z[d] = zd;
         part_sums(own ? rd * zd : 0.0, own ? rd * rd : 0.0, 2, parts + nparts);
-        if (!(ok = grid_barrier(&st->bar, ++epoch * gridDim.x, &st->bar_err))) break;
+        if (!(ok = grid_barrier(&st->wait.bar, ++epoch * gridDim.x, &st->wait.err, polls))) break;
         double t2[2];
         coop_total<2>(parts + nparts, nparts, sh2, t2);
         coop_beta(s, t2[0], t2[1], eps, tolSq, maxIter, st, blockIdx.x == 0 && tid == 0);

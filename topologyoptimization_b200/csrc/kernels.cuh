@@ -140,7 +140,7 @@ __global__ void __launch_bounds__(kOcThreads) k_oc_bisect(const float *x, const 
                                                           const uint8_t *__restrict__ pres,
                                                           const uint8_t *__restrict__ voidm, long long n, long long per,
                                                           int cap, double volfrac, double move, int max_bisections,
-                                                          OCState *s, const float *xold, float *xnew);
+                                                          OCState *s, const float *xold, float *xnew, unsigned polls);
 
 __global__ void k_energy_wgsl(const float *__restrict__ U, const float *__restrict__ KE,
                               const int32_t *__restrict__ edofs, int nel, int es, float *__restrict__ out);
@@ -174,7 +174,7 @@ __global__ void __launch_bounds__(kCoop2Threads) k_cg_coop2(const double *__rest
                                                             const double *__restrict__ invD,
                                                             const uint8_t *__restrict__ fixed, double *U, double *r,
                                                             double *z, double *pa, double *pb, CGState *st,
-                                                            double *parts);
+                                                            double *parts, int iters, unsigned polls);
 __global__ void k_cg_abs_tol(CGState *st, double tol);
 
 }  // namespace tpo

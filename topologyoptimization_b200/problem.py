@@ -65,6 +65,11 @@ class Problem:
         raw = None if stream is None else getattr(stream, "cuda_stream", stream)
         N.check(N.lib().tpo_set_stream(self.h, C.c_void_p(raw) if raw else None), "tpo_set_stream")
 
+    def set_launch_limits(self, iterations=4096, polls=1 << 22):
+        """Limits of the kernels that run a whole loop on the device: PCG iterations of one
+        launch (even) and polls of a wait inside it before the call raises TPO_TIMEOUT."""
+        N.check(N.lib().tpo_set_launch_limits(self.h, int(iterations), int(polls)), "tpo_set_launch_limits")
+
     # ---- operators ------------------------------------------------------------------
     def set_densities(self, x, penal, E0=1.0, Emin=1e-9):
         if hasattr(x, "is_cuda") and x.is_cuda:
