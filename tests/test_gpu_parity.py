@@ -796,3 +796,44 @@ def test_oc_unreachable_volume_keeps_masks(native, oracle, dims, volfrac, share_
         xn = d_xn.cpu().numpy()
     assert nb == nbr and lm == lmr
     assert np.array_equal(xn, xr, equal_nan=True)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dims,general", [((60, 20, 4), False), ((300, 100, 4), False), ((2000, 4, 4), False),
+                                          ((4, 300, 100), False), ((60, 20, 4), True), ((96, 48, 48), True),
+                                          ((300, 100, 4), True)])
+def test_thin_grid_apply(native, oracle, dims, general):
+    """Grids that are thin on one or two axes, whose share of the small-grid apply's columns
+    decides between it (one plane a block, two) and the strip kernel, and an FP32-rounded Ke
+    (the general form) with each of the three: K u in FP64 and FP32, and three PCG iterations
+    (fused reductions).  Bounds of the suite's other applies (1e-12, 2e-6) and solves (1e-10)."""
+    import torch
+    from topologyoptimization_b200 import Problem, mesh
+    rng = np.random.default_rng(13)
+    fixed = mesh.fixed_mask(*dims, "left")
+    Ke = oracle.lk(0.3)
+    if general:
+        Ke = Ke.astype(np.float32).astype(np.float64)
+    x = rng.uniform(0.3, 1.0, int(np.prod(dims))).astype(np.float32)
+    x[rng.random(x.size) < 0.1] = 1e-3
+    u = rng.standard_normal(len(fixed))
+    E = 1e-9 + x.astype(np.float64) ** 3 * (1 - 1e-9)
+    act = np.flatnonzero(E > 1e-6).astype(np.int32)
+    ref = oracle.apply_a(Ke, oracle.edofs3d(*dims), E, act, u)
+    with Problem(*dims, fixed, Ke=Ke if general else None) as P:
+        P.set_densities(x, 3.0)
+        assert rel_inf(P.apply(u), ref) < 1e-12
+        d_u, d_o = _dev(u.astype(np.float32)), torch.empty(len(u), dtype=torch.float32, device="cuda")
+        P.apply_f32_dev(d_u, d_o)
+        torch.cuda.synchronize()
+        assert rel_inf(d_o.cpu().numpy(), ref) < 2e-6
+        if general:
+            return
+        F = u * (fixed == 0)
+        P.set_load(F)
+        U, info = P.solve(None, precond=native.PREC_MG, max_iter=3, tol=0.0, warm_start=0, ref_epsilon=1)
+    mg = oracle.MG(*dims, Ke, fixed)
+    mg.update(x, 3.0)
+    Uo, ito = mg.mgpcg(F, 3, 0.0)
+    assert info.iterations == ito == 3
+    assert rel_inf(U, Uo) < 1e-10

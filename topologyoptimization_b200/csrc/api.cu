@@ -360,18 +360,67 @@ void configure_apply(size_t smem) {
     if (apply_conc<T, Epi>() == 0 || conc < apply_conc<T, Epi>()) apply_conc<T, Epi>() = conc;
 }
 
-// Node planes per CTA of the small-grid kernel, 0: the strip kernel.  Measured back to back in a
-// graph (us, FP64 / FP32; strip, one plane, two planes):
-//     16x8x8        1.4e3 nodes    5.7 / 6.2     3.1 / 2.8     3.8 / 3.3
-//     64x32x32      7.1e4          8.1 / 6.6     5.3 / 4.6     5.7 / 4.7
-//     75x37x39      1.2e5          9.9 / 8.5     8.8 / 6.8     9.6 / 5.8
-//     96x48x48      2.3e5         13.3 / 8.7    12.7 / 9.2    11.1 / 7.3
-//     110x52x58     3.5e5         15.2 / 10.6   21.4 / 14.1   18.9 / 11.9
-// The node count of a batched launch is that of all its right-hand sides.
-inline int small_planes(const Grid &g, int nrhs) {
-    const long long n = g.nnodes * nrhs;
-    if (g.nnx > 8192) return 0;  // blocks along x
-    return n <= 90000 ? 1 : (n <= 280000 ? 2 : 0);
+// A grid with what the choice between the two kernels needs, beside the Grid that kernels take: CTAs
+// of the small-grid kernel at one plane each, CTAs of the strip kernel's launch by the cost
+// model (FP32, FP64; one per SM resident) and the planes each runs through.
+struct PlannedGrid : Grid {
+    int small_ctas = 0, strip_ctas[2] = {0, 0}, strip_planes[2] = {0, 0};
+    template <typename T>
+    void plan_strip() {
+        if (walsh_out_cols<T>(nnz) <= 0) return;  // refused by configure_all_applies
+        const ApplyShape s = apply_shape<T>(*this, g_num_sms ? g_num_sms : 148);
+        const int i = sizeof(T) == 8 ? 1 : 0;
+        strip_ctas[i] = (int)(s.grid.x * s.grid.y);
+        strip_planes[i] = s.xchunk + 1;
+    }
+    PlannedGrid() = default;
+    PlannedGrid(int nelx, int nely, int nelz) : Grid(make_grid(nelx, nely, nelz)) {
+        const dim3 sg = small_grid(*this, 1, 1);
+        small_ctas = (int)(sg.x * sg.y);
+        plan_strip<float>();
+        plan_strip<double>();
+    }
+};
+
+// Node planes per CTA of the small-grid kernel, 0: the strip kernel.  The small-grid kernel's time
+// follows its CTAs, whatever share of their 8 x 16 columns the grid fills (0.0055 us each in
+// FP64, 0.0035 in FP32, above some 600 of them); the strip kernel packs columns along the line
+// and takes 2 us and 2 us more for each plane that its CTAs run through, over all waves.  The
+// lines lie where the two meet: 340 (FP64) and 620 (FP32) CTAs of one plane for each such plane.
+// Two planes a CTA are faster from two waves of one-plane CTAs on: 1184 (four an SM) in FP64; in FP32
+// 1036 (146 against 149 us a PCG iteration at 75x37x39, where the plain apply alone says
+// otherwise).  Measured back to back in a graph (us, FP64 | FP32; strip, one plane, two planes;
+// * the rule's choice):
+//                    CTAs   planes
+//     16x8x8           17   2, 2     5.8  2.7* 3.5 |  6.2  2.3* 3.0
+//     64x32x32        520   3, 2     8.1  4.8* 5.9 |  6.5  4.2* 4.3
+//     48x48x48        882   3, 2     9.8  7.6* 7.4 |  6.5  6.3* 6.8
+//     75x37x39       1140   4, 3     9.8  8.4* 9.2 |  8.4  6.3  6.9*
+//     96x48x48       1746   6, 3    13.2 12.2 10.6*|  8.6  8.6  6.9*
+//     60x60x60       1952   5, 3    11.6*14.2 13.2 |  8.6* 9.4  9.0
+//     110x52x58      3108   7, 4    15.0*20.9 18.4 | 10.5*13.6 11.5
+//     60x20x4         183   2, 2     5.8  3.7* 4.2 |  6.2  3.1* 3.6
+//     100x100x3      1313   2, 2     6.3*10.1  9.6 |  6.2* 7.1  6.7
+//     300x4x100      2107   6, 4    13.2*12.8 11.7 |  9.9  9.2  7.8*
+//     4x300x100      1330   6, 3    13.0 10.3  9.6*|  8.4  6.9  6.8*
+//     300x100x4      3913   4, 4    10.0*24.4 21.7 |  9.9*16.1 13.3
+//     200x200x3      5025   4, 3    10.0*30.6 26.5 |  8.4*20.2 16.4
+//     2000x4x4       2001  15, 15   25.6 12.1 10.9*| 28.4  8.7  7.4*
+// A line at 280,000 nodes sent the thin ones among these to the small-grid kernel: a V-cycle PCG
+// iteration on 200x200x3 (FP64 / FP32 cycle) took 1342 / 694 us with it and takes 399 / 343, on
+// 300x100x4 511 / 384 and 404 / 336, on 60x60x60 230 / 178 and 180 / 163.  A batched launch has the
+// CTAs of all its right-hand sides in both kernels: FP64 iterations with strip / one / two planes
+// on all levels: 8 x 40x20x20 221 / 203 / 210, 32 x 32x16x16 441 / 249 / 255, 4 x 64x32x32
+// 271 / 240 / 251, 8 x 100x100x3 1174 / 2321 / 2689.
+template <typename T>
+inline int small_planes(const PlannedGrid &g, int nrhs) {
+    constexpr int i = sizeof(T) == 8 ? 1 : 0;
+    constexpr long long kCtasPerPlane = i ? 340 : 620;
+    const int sms = g_num_sms ? g_num_sms : 148;
+    const long long ctas = (long long)g.small_ctas * nrhs, strip = (long long)g.strip_ctas[i] * nrhs;
+    const long long waves = strip <= sms ? 1 : (strip + sms - 1) / sms;
+    if (g.nnx > 8192 || ctas > kCtasPerPlane * waves * g.strip_planes[i]) return 0;  // (blocks along x)
+    return ctas <= (i ? 1184 : 1036) ? 1 : 2;
 }
 template <typename T, class Epi, bool kGeneral>
 void launch_small(cudaStream_t st, const Grid &g, int tx, const WalshKe<T> &wk, const T *p, const T *Eact,
@@ -382,9 +431,9 @@ void launch_small(cudaStream_t st, const Grid &g, int tx, const WalshKe<T> &wk, 
 }
 
 template <typename T, class Epi>
-void launch_apply(cudaStream_t st, const Grid &g, const WalshKe<T> &wk, const T *p, const T *Eact, const Epi &epi,
+void launch_apply(cudaStream_t st, const PlannedGrid &g, const WalshKe<T> &wk, const T *p, const T *Eact, const Epi &epi,
                   const CGState *cg, int nrhs = 1) {
-    if (const int tx = small_planes(g, nrhs)) {
+    if (const int tx = small_planes<T>(g, nrhs)) {
         if constexpr (std::is_same_v<T, double>) {
             if (wk.general) {
                 launch_small<T, Epi, true>(st, g, tx, wk, p, Eact, epi, cg, nrhs);
@@ -578,7 +627,7 @@ constexpr int kModeF32Bf16 = 11;  // FP64 PCG, FP32 V-cycle with BF16 tensor-cor
 constexpr int kIterModes = 2 * kModeStride;
 
 struct Level {
-    Grid g{};
+    PlannedGrid g;
     bool dense = false;
     uint8_t *fixed = nullptr;
     double *E = nullptr, *Eact = nullptr, *invD = nullptr;
@@ -619,7 +668,7 @@ struct tpo_batch {
 };
 
 struct tpo_problem {
-    Grid g{};
+    PlannedGrid g;
     int nl = 0;
     Level L[kMaxLevels];
     tpo_mg_opts mg{};
@@ -779,7 +828,7 @@ void build_levels(tpo_problem *P) {
     for (int li = 1; li < maxl; li++) {
         const int nx = cx / 2, ny = cy / 2, nz = cz / 2;
         if (nx < 2 || ny < 2 || nz < 2) break;
-        P->L[li].g = make_grid(nx, ny, nz);
+        P->L[li].g = PlannedGrid(nx, ny, nz);
         P->nl++;
         cx = nx; cy = ny; cz = nz;
     }
@@ -1019,9 +1068,9 @@ void tune_apply_shapes(tpo_problem *P) {
     if (cs != cudaStreamCaptureStatusNone) return;  // timing needs an uncaptured stream
     for (int li = 0; li < P->nl; li++) {
         Level &L = P->L[li];
-        if (L.dense || small_planes(L.g, 1)) continue;
-        tune_apply_shape<float>(P, L);
-        tune_apply_shape<double>(P, L);
+        if (L.dense) continue;
+        if (!small_planes<float>(L.g, 1)) tune_apply_shape<float>(P, L);
+        if (!small_planes<double>(L.g, 1)) tune_apply_shape<double>(P, L);
     }
     P->g.nch[0] = P->L[0].g.nch[0];  // the fine grid's copy used by the single-apply entries
     P->g.nch[1] = P->L[0].g.nch[1];
@@ -1606,7 +1655,7 @@ tpo_problem *create_problem(const tpo_grid *gr, const double *Ke, double nu, con
     check_device();
     if (!gr || gr->nelx < 1 || gr->nely < 1 || gr->nelz < 1) fail(TPO_BAD_ARG, "grid must be at least 1x1x1");
     if (!fixed) fail(TPO_BAD_ARG, "fixedMask is null");
-    const Grid g = make_grid(gr->nelx, gr->nely, gr->nelz);
+    const PlannedGrid g(gr->nelx, gr->nely, gr->nelz);
     if (g.ndof > (1LL << 31) - 1) fail(TPO_BAD_ARG, "grid too large for 32-bit DOF indices");
     tpo_problem *P = new tpo_problem();
     try {
@@ -1645,10 +1694,7 @@ tpo_problem *create_problem(const tpo_grid *gr, const double *Ke, double nu, con
         const long long tc_tiles = (long long)((g.nny + kTcNodesY - 1) / kTcNodesY) * ((g.nnz + kTcNodesZ - 1) / kTcNodesZ);
         const size_t colb = (size_t)std::max((ncol + tout - 1) / tout, tc_tiles);
         size_t blocks = std::max<size_t>(4096, colb * (size_t)std::min(g.nnx, 512));
-        if (small_planes(g, 1)) {
-            const dim3 sg = small_grid(g, 1, 1);
-            blocks = std::max(blocks, (size_t)sg.x * sg.y);
-        }
+        if (small_planes<float>(g, 1) || small_planes<double>(g, 1)) blocks = std::max(blocks, (size_t)g.small_ctas);
         P->npartials = 2 * blocks;
         P->partials = dalloc<double>(P->npartials);
         P->st = dalloc<CGState>(1);
