@@ -837,3 +837,51 @@ def test_thin_grid_apply(native, oracle, dims, general):
     Uo, ito = mg.mgpcg(F, 3, 0.0)
     assert info.iterations == ito == 3
     assert rel_inf(U, Uo) < 1e-10
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dims,least", [((4, 4, 4), 1), ((14, 4, 4), 1), ((12, 6, 6), 7), ((14, 6, 6), 7), ((16, 6, 6), None)])
+def test_coarse_sweeps_or_matrix(native, oracle, dims, least):
+    """Coarsest levels of 81, 216, 336, 384 and 432 DOFs: a single V-cycle on new moduli, and a solve
+    of fewer iterations than `least`, run the 32 sweeps; a longer solve forms their matrix, and
+    what follows on the same moduli takes it (counted by launches).  Above 384 DOFs only sweeps.
+    Within the other V-cycles' and solves' 1e-11 and 1e-10 of the oracle either way."""
+    from topologyoptimization_b200 import Problem, mesh
+    fixed = mesh.fixed_mask(*dims, "left")
+    rng = np.random.default_rng(14)
+    x = rng.uniform(0.3, 1.0, int(np.prod(dims))).astype(np.float32)
+    b = rng.standard_normal(len(fixed)) * (fixed == 0)
+    mg = oracle.MG(*dims, oracle.lk(0.3), fixed, max_levels=2)
+    count = native.lib().tpo_launch_count
+
+    def vcycle(P):
+        n0 = count()
+        z = P.vcycle(b)
+        assert rel_inf(z, mg.vcycle(b)) < 1e-11
+        return count() - n0
+
+    def solve(P, n):
+        n0 = count()
+        U, info = P.solve(None, precond=native.PREC_MG, max_iter=n, tol=0.0, warm_start=0, ref_epsilon=1)
+        Uo, ito = mg.mgpcg(b, n, 0.0)
+        assert info.iterations == ito == n and rel_inf(U, Uo) < 1e-10
+        return count() - n0
+
+    with Problem(*dims, fixed, mg=native.default_mg_opts(max_levels=2)) as P:
+        P.set_load(b)
+        for s in (x, 1.0 - 0.5 * x):  # the second time over, graphs of the first exist
+            P.set_densities(s, 3.0)
+            mg.update(s, 3.0)
+            sweeps = vcycle(P)
+            assert sweeps > 30
+            if least is None:
+                solve(P, 8)
+                assert vcycle(P) == sweeps
+                continue
+            if least > 1:
+                solve(P, least - 1)
+                assert vcycle(P) == sweeps
+            solve(P, least)
+            assert vcycle(P) < sweeps - 25
+            solve(P, 2)
+            assert vcycle(P) < sweeps - 25

@@ -625,6 +625,7 @@ constexpr int kModeStride = 12;
 constexpr int kModeBddc = 10;
 constexpr int kModeF32Bf16 = 11;  // FP64 PCG, FP32 V-cycle with BF16 tensor-core fine-level applies
 constexpr int kIterModes = 2 * kModeStride;
+constexpr int kIterGraphs = 2 * kIterModes;  // kIterModes more: the coarsest level by its sweeps although it has S
 
 struct Level {
     PlannedGrid g;
@@ -732,9 +733,10 @@ struct tpo_problem {
     int coop_iters = kCoopIters;
     unsigned wait_polls = kBarrierPolls;
     // captured PCG iteration chunks
-    cudaGraphExec_t gexec[kIterModes] = {};
-    int gchunk[kIterModes] = {};
-    long long gnodes[kIterModes] = {};
+    bool poly = false;  // the running call takes the coarsest level's sweeps as their matrix S
+    cudaGraphExec_t gexec[kIterGraphs] = {};
+    int gchunk[kIterGraphs] = {};
+    long long gnodes[kIterGraphs] = {};
 };
 
 namespace {
@@ -860,8 +862,7 @@ void build_levels(tpo_problem *P) {
     }
     if (maxT) P->Ttmp = dalloc<double>(maxT);
     {
-        // Sweeps as a matrix: from 4 sweeps on, up to kPolyMaxN DOFs (675, the coarsest level of
-        // a 256x128x128 grid), where forming it stays below the time of five V-cycles' sweeps.
+        // Sweeps as a matrix: from 4 sweeps on, up to kPolyMaxN DOFs (choose_coarse_poly says when).
         Level &C = P->L[P->nl - 1];
         if (C.dense && !o.coarse_direct && o.nu1 + o.coarse_iters >= 4 && C.g.ndof <= kPolyMaxN) {
             C.S = dalloc<double>((size_t)C.g.ndof * C.g.ndof);
@@ -1141,18 +1142,26 @@ void residual(tpo_problem *P, int li, const T *b, const T *x, T *res, const CGSt
     }
 }
 
-// The matrix of the coarsest level's sweeps for the current moduli.  Called before a V-cycle is
-// launched or captured: never inside a capture.
-void ensure_coarse_poly(tpo_problem *P) {
+// Whether the V-cycles of this call, `cycles` of them at most, take the coarsest level's sweeps as
+// their matrix S, which is formed here if need be.  Called before a V-cycle is launched or
+// captured: never inside a capture.  Forming takes 62, 110, 170, 550, 2070 us at 81, 135, 216,
+// 336, 675 DOFs (two columns a block: a second wave of blocks from 297 on) and saves some 72 us
+// a V-cycle at all of them, so it pays from 1, 2, 2, 8 and 28 V-cycles on: kPolyMaxN lies between
+// the last two, and a call that can make fewer runs the sweeps.  (Formed always, a solve of two
+// iterations took 1149 in place of 877 us at 96x48x48, 2452 in place of 637 with 675 DOFs.  What a
+// warm start saves is not known beforehand: one that ends before eight V-cycles pays up to 0.5 ms.)
+void choose_coarse_poly(tpo_problem *P, int cycles) {
     Level &C = P->L[P->nl - 1];
-    if (!C.S || C.S_version == P->E_version) return;
-    const int n = (int)C.g.ndof;
-    k_coarse_pack<<<nblk(81LL * n), 256, 0, P->s>>>(C.K, C.g, C.Sk);
-    CKL();
-    k_coarse_poly<<<nblk(n, 2), 1024, coarse_poly_smem(n), P->s>>>(C.Sk, C.g, C.invD, C.fixed, C.omega, C.womega,
-                                                                  P->mg.nu1 + P->mg.coarse_iters, C.S);
-    CKL();
-    C.S_version = P->E_version;
+    if (C.S && C.S_version != P->E_version && cycles >= (C.g.ndof <= 216 ? 2 : 8)) {
+        const int n = (int)C.g.ndof;
+        k_coarse_pack<<<nblk(81LL * n), 256, 0, P->s>>>(C.K, C.g, C.Sk);
+        CKL();
+        k_coarse_poly<<<nblk(n, 2), 1024, coarse_poly_smem(n), P->s>>>(C.Sk, C.g, C.invD, C.fixed, C.omega, C.womega,
+                                                                      P->mg.nu1 + P->mg.coarse_iters, C.S);
+        CKL();
+        C.S_version = P->E_version;
+    }
+    P->poly = C.S && C.S_version == P->E_version;
 }
 
 // x must be treated as zero on entry (it is fully overwritten).
@@ -1162,7 +1171,7 @@ template <typename T>
 bool vcycle(tpo_problem *P, int li, const T *b, T *x, const CGState *st, const double *rdot = nullptr) {
     Level &L = P->L[li];
     const bool last = li == P->nl - 1;
-    if (last && (L.Kinv || L.S)) {  // direct coarse solve (x = K^-1 b on the free DOFs) or the sweeps' matrix
+    if (last && (L.Kinv || (L.S && P->poly))) {  // direct coarse solve (x = K^-1 b on the free DOFs) or the sweeps' matrix
         const int n = (int)L.g.ndof;
         Chain{G(P, (n + 7) / 8), 256, 0, P->s}(k_dense_mv<T>, L.Kinv ? L.Kinv : L.S, n, b, x, st);
         return false;
@@ -1416,7 +1425,7 @@ void enqueue_iteration(tpo_problem *P, int mode) {
     Chain{G(P, pair_blocks(n)), 256, 0, P->s}(k_cg_p, P->p, P->z, n, P->st);
 }
 
-cudaGraphExec_t get_iteration_graph(tpo_problem *P, int mode, int chunk) {
+cudaGraphExec_t get_iteration_graph(tpo_problem *P, int mode, int chunk) {  // mode: an index of gexec
     if (P->gexec[mode] && P->gchunk[mode] == chunk) return P->gexec[mode];
     if (P->gexec[mode]) {
         cudaGraphExecDestroy(P->gexec[mode]);
@@ -1447,6 +1456,7 @@ cudaGraphExec_t get_iteration_graph(tpo_problem *P, int mode, int chunk) {
 // Replays chunks of captured iterations until the device state says done.
 void run_iterations(tpo_problem *P, int mode, CGState *st, CGState *st_host, int max_iter) {
     const int chunk = mode == 1 ? 16 : 4;
+    if (P->L[P->nl - 1].S && !P->poly) mode += kIterModes;
     cudaGraphExec_t ge = get_iteration_graph(P, mode, chunk);
     const long long max_launch = (std::max(0, max_iter) + chunk - 1) / chunk + 1;
     for (long long c = 0;; c++) {
@@ -1543,7 +1553,8 @@ void solve_fp64(tpo_problem *P, const tpo_solve_opts &o, tpo_solve_info *info) {
         P->use_tc_cg = false;
         P->tc_mode = o.tensor_cores >= 5 ? 2 : (o.tensor_cores >= 3 ? 1 : 0);
     }
-    if (o.precond == TPO_PREC_MG) ensure_coarse_poly(P);
+    if (o.precond == TPO_PREC_MG) choose_coarse_poly(P, std::min(o.max_iter, 1 << 30) + 1);
+    else P->poly = true;  // no V-cycle in its iterations: one graph
     if (o.precond == TPO_PREC_BDDC) {
         if (P->nrhs > 1) fail(TPO_BAD_ARG, "the BDDC preconditioner solves one right-hand side at a time");
         if (P->bddc_iters != o.bddc_smoother_iters && P->gexec[kModeBddc]) {  // captured with another count
@@ -1607,7 +1618,7 @@ void solve_fp64(tpo_problem *P, const tpo_solve_opts &o, tpo_solve_info *info) {
 void solve_mixed(tpo_problem *P, const tpo_solve_opts &o, tpo_solve_info *info) {
     if (!P->have_E) fail(TPO_BAD_ARG, "tpo_solve: densities were never set");
     ensure_mixed(P);
-    ensure_coarse_poly(P);
+    choose_coarse_poly(P, std::min(o.max_iter, 1 << 30) + 1);
     P->use_tc = o.tensor_cores >= 1;
     P->use_tc_cg = o.tensor_cores == 2 || o.tensor_cores == 4;
     P->tc_mode = o.tensor_cores >= 3 ? 1 : 0;
@@ -2075,7 +2086,7 @@ tpo_status tpo_vcycle(tpo_problem *p, const double *b, double *z) {
         if (!p || !b || !z) fail(TPO_BAD_ARG, "null argument");
         if (!p->have_E) fail(TPO_BAD_ARG, "densities were never set");
         const size_t nb = (size_t)p->g.ndof * sizeof(double);
-        ensure_coarse_poly(p);
+        choose_coarse_poly(p, 1);
         CK(cudaMemcpyAsync(p->r, b, nb, cudaMemcpyHostToDevice, p->s));
         vcycle<double>(p, 0, p->r, p->z, nullptr);
         CK(cudaMemcpyAsync(z, p->z, nb, cudaMemcpyDeviceToHost, p->s));
@@ -2280,7 +2291,8 @@ namespace {
 void ensure_batch(tpo_problem *P, int nb, bool f32) {
     if (P->batch && P->batch->nb == nb && (P->batch->f32 || !f32)) return;
     batch_free(P);
-    for (int m = kModeStride; m < kIterModes; m++) {  // graphs captured on the previous batch buffers
+    for (int m = 0; m < kIterGraphs; m++) {  // graphs captured on the previous batch buffers
+        if (m / kModeStride % 2 == 0) continue;
         if (P->gexec[m]) cudaGraphExecDestroy(P->gexec[m]);
         P->gexec[m] = nullptr;
         P->gchunk[m] = 0;
@@ -2445,7 +2457,7 @@ tpo_status tpo_set_spring(tpo_problem *p, int64_t dof, double k) {
         p->g.sdof = p->L[0].g.sdof = dof;
         p->g.sk = p->L[0].g.sk = kk;
         // captured iterations hold the grid by value: capture them again
-        for (int m = 0; m < kIterModes; m++) {
+        for (int m = 0; m < kIterGraphs; m++) {
             if (p->gexec[m]) cudaGraphExecDestroy(p->gexec[m]);
             p->gexec[m] = nullptr;
             p->gchunk[m] = 0;

@@ -408,10 +408,10 @@ __global__ void k_coarse_mask_inverse(const double *__restrict__ Ainv, int n, co
 
 // ---- coarsest level: its sweeps as one matrix -----------------------------------------
 // The reference solves the coarsest level by nu1 + 30 damped Jacobi sweeps from zero, a linear
-// map of b: x = S b.  S is formed once per hierarchy update, column by column (the sweeps on
-// b = e_c), and a V-cycle then needs one matrix-vector product there instead of 31 launches
-// (about 3 us each at 135 and 216 DOFs, half of a V-cycle's time on the worker's grids; S
-// itself takes 168 us at 216 DOFs).
+// map of b: x = S b.  S is formed at most once per hierarchy update, column by column (the sweeps
+// on b = e_c), and a V-cycle then needs one matrix-vector product there instead of 31 launches
+// (about 72 us less, half of a V-cycle's time on the worker's grids; choose_coarse_poly of api.cu
+// has what forming S takes and when it pays).
 //
 // The operator's stencil entries, 81 a row (the order of dense_row_dot), 0 outside the grid.
 __global__ void k_coarse_pack(const double *__restrict__ K, const Grid g, double *__restrict__ Ks) {

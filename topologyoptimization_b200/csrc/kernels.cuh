@@ -51,7 +51,7 @@ __global__ void k_dense_rows(const double *__restrict__ K, const Grid g, const u
 __global__ void k_dense_matvec_seq(const double *__restrict__ K, int n, const double *__restrict__ p,
                                    double *__restrict__ Ap);
 // coarsest level: its Jacobi sweeps from zero as a matrix
-constexpr int kPolyMaxN = 704;  // largest level that takes this form
+constexpr int kPolyMaxN = 384;  // largest level that takes this form (choose_coarse_poly of api.cu)
 inline size_t coarse_poly_smem(int n) { return (size_t)n * (2 * sizeof(double2) + 81 * sizeof(unsigned short)); }
 __global__ void k_coarse_pack(const double *__restrict__ K, const Grid g, double *__restrict__ Ks);
 __global__ void __launch_bounds__(1024) k_coarse_poly(const double *__restrict__ Ks, const Grid g,
