@@ -63,7 +63,7 @@ std::atomic<long long> g_launches{0};
 // started, and waits there for its results, so that a launch's 1 to 2 us of start-up is hidden.
 // Microseconds an iteration before -> after, with the FP32 / FP64 cycle: 94 / 97 -> 85 / 87 at
 // 32x16x16, 128 / 140 -> 120 / 132 at 64x32x32, 170 / 202 -> 167 / 200 at 96x48x48, 337 / 437
-// -> 327 / 428 at 150x74x78, 1057 / 1485 -> 1048 / 1478 at 256x128x128.
+// -> 325 / 427 at 150x74x78, 1057 / 1485 -> 1048 / 1478 at 256x128x128.
 struct Chain {
     dim3 grid, block;
     size_t smem;
@@ -1498,7 +1498,8 @@ inline long long coop_resident(const void *kernel, int threads, size_t smem) {
 
 // Jacobi-PCG of a small problem in one launch: up to 192 nodes per SM (28,416 on 148 SMs).  At
 // 30x10x10 an iteration takes 6.3 us instead of 18.6 (graph of three launches), at 17,199 nodes
-// 9.1 instead of 19.3, at the limit 10.2 instead of 19.4.  False when the problem is too large for it.
+// 9.1 instead of 19.3, at the limit 10.2 instead of 19.4: the limit is the largest form that is
+// compiled (six nodes a lane), not where this stops paying.  False when the problem is too large.
 bool jacobi_coop(tpo_problem *P, int max_iter) {
     const Grid &g = P->L[0].g;
     const long long sms = g_num_sms ? g_num_sms : 148;

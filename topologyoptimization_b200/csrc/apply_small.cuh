@@ -7,9 +7,11 @@
 // (node planes, moduli and the epilogue's operands), each thread runs its element column
 // through the box's planes in registers, and two barriers separate load, transform and sum.
 // The operations of an element and the order of a node's four contributions are the strip
-// kernel's, so both give the same bits in FP32 (packed and scalar arithmetic round alike) and
-// which one runs is a matter of time only (the table is at the rule, small_planes).  What is
-// left is a launch's own 2 us and one round of loads, transforms and stores.
+// kernel's, so K u has the same bits from both (in FP32 packed and scalar arithmetic round
+// alike).  A fused dot product is added up by other blocks: launches with one differ in its
+// rounding, and a batched solve, which may take the other kernel, can differ from a single one
+// there.  The rule that chooses and its table are at small_planes.  What is left is a launch's
+// own 2 us and one round of loads, transforms and stores.
 #pragma once
 #include "apply_walsh.cuh"
 

@@ -13,6 +13,12 @@
 //      -- barrier, every block adds up all parts: beta, the stop test
 // All blocks take the same decisions from the same numbers.  p alternates between two arrays, so
 // that no block overwrites a value another still reads.
+//
+// Cooperative launches of several streams run one after the other, where separate launches ran
+// side by side.  300 iterations on each of 1, 2, 4, 8 handles with a thread each took, as separate
+// launches and as one: 5.7, 6.1, 6.4, 9.0 and 1.9, 2.9, 5.4, 10.9 ms at 30x10x10; 6.0, 6.3, 7.6,
+// 13.2 and 3.1, 6.1, 12.2, 24.2 ms at 60x20x20.  Up to two solves at a time gain or lose nothing;
+// from four on at 60x20x20 (eight at 30x10x10) they lose.
 #pragma once
 #include "common.cuh"
 

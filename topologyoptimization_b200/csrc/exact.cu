@@ -576,8 +576,11 @@ __device__ __forceinline__ int oc_bits(const OcElem &e, double rl) {
 // between its limits, and every block adding up all blocks' words, a call of nine steps took
 // 74, 112, 210, 347 us for 24,000, 524,288, 2.05M and 4.2M elements; it takes 67, 80, 118, 234
 // (the last keeps only half of its elements in shared memory).  Several steps a pass take the
-// design update of 2.05M elements (some 40 steps, all kernels) from 0.82 to 0.75 ms; beyond
-// kOcAheadMax the steps that are dropped cost more than the barriers that are saved.
+// design update of 2.05M elements (some 40 steps, all kernels) from 0.82 to 0.75 ms.  The steps
+// that are dropped at the end cost as much as the barriers saved near kOcAheadMax: calls of 49
+// and 32 steps, one at a time / four, take 945 / 884 and 637 / 625 us with 28,340 elements a block,
+// 1216 / 1157 and 815 / 810 with 35,425, 1991 / 1940 and 1327 / 1349 with 55,352, 2612 / 2561 and
+// 1745 / 1805 with 70,850.
 __global__ void __launch_bounds__(kOcThreads) k_oc_bisect(const float *x, const float *dc,
                                                           const uint8_t *__restrict__ pres,
                                                           const uint8_t *__restrict__ voidm, long long n, long long per,
