@@ -373,7 +373,7 @@ struct PlannedGrid : Grid {
         strip_ctas[i] = (int)(s.grid.x * s.grid.y);
         strip_planes[i] = s.xchunk + 1;
     }
-    PlannedGrid() = default;
+    PlannedGrid() : Grid{} {}
     PlannedGrid(int nelx, int nely, int nelz) : Grid(make_grid(nelx, nely, nelz)) {
         const dim3 sg = small_grid(*this, 1, 1);
         small_ctas = (int)(sg.x * sg.y);
